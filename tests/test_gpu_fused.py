@@ -217,3 +217,30 @@ def test_line_sweep_shapes(gpu_lib, monkeypatch, name, mk, lim, bc, n, tweak):
     and 32-row chunks unevenly (one strip, partly filled strips, fewer rows
     than a chunk, several chunks), against the oracle and the split kernels."""
     test_fused_against_oracle_and_split(gpu_lib, monkeypatch, name, mk, lim, bc, n, tweak)
+
+
+@pytest.mark.parametrize("nx,lim,bc", [((33, 33, 33), "minmod", "symm"),
+                                       ((20, 9, 7), "woodward", "cont"),
+                                       ((64, 50, 41), "woodward", "periodic"),
+                                       ((97, 88, 90), "minmod", "cont")])
+def test_z_chunk_by_size_is_invisible(gpu_lib, monkeypatch, nx, lim, bc):
+    """The z chunk that a small grid gets by its size (2 to 8 planes, a last
+    chunk of one plane among them) gives the bits of one pinned at 32."""
+    s = inistate.random_modes(max(nx), seed=6, p0=0.5)
+    s.x = inistate.domain_grid(nx, (0.0,) * 3, tuple(n / max(nx) for n in nx))
+    s.w = np.ascontiguousarray(s.w[:, :nx[0], :nx[1], :nx[2]])
+    s.nx = nx
+    p = inistate.params_for(s, limiter=lim, bc=bc, precision=abi.PREC_MIXED)
+    if bc == "symm":
+        reflecting(p, 3)
+    out = []
+    for pin in (None, "32"):
+        if pin:
+            monkeypatch.setenv("VACGPU_NZC", pin)
+        e = Engine(p, s.x, s.w)
+        e.step(5)
+        assert e.kernel_stats()["sweep"][0] == 15
+        out.append((e.t, e.state()))
+        e.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1].view(np.uint64), out[1][1].view(np.uint64))

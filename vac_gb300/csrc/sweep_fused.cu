@@ -8,7 +8,7 @@ namespace vacgpu {
 
 int fused_smem_bytes(int nw, int k) { return fused_smem_floats(nw, k) * 4; }
 
-bool launch_sweep_pair(const FusedArgs& a, int D, bool mhd, const void* tmap, int nzc,
+bool launch_sweep_pair(FusedArgs a, int D, bool mhd, const void* tmap, int nzc,
                        cudaStream_t st);
 bool launch_sweep_line2(const FusedArgs& a, const float* win, int D, bool mhd,
                         cudaStream_t st);
@@ -78,7 +78,6 @@ bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win, 
   }
   a.ctrl = s.ctrl;
   a.wout = wout;
-  a.nzc = nzc;
   for (int d = 0; d < 3; d++) a.gravf[d] = (float)s.ph.src_par[d];
   a.cfl = s.ph.courantpar > 0.0;
   const int nw = s.mhd ? 2 + 2 * s.ndir : 2 + s.ndir;
@@ -88,7 +87,16 @@ bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win, 
       if (s.ph.typeB[2 * d][v] == VACGPU_BC_ASYMM) a.asymm_lo[d] |= 1 << v;
       if (s.ph.typeB[2 * d + 1][v] == VACGPU_BC_ASYMM) a.asymm_hi[d] |= 1 << v;
     }
-  // tiles over x and the row axis, z chunks along the marching axis
+  // 3-D grids: the two-cells-per-thread kernel (packed FP32) where it
+  // applies; VACGPU_PAIR=0 keeps the one-cell kernel
+  if (nd == 3 && launch_sweep_pair(a, s.d0, s.mhd, tmap, nzc, st))
+    return true;
+  // 2-D grids: the warp-marching two-cells-per-thread kernel where it applies
+  if (nd == 2 && launch_sweep_line2(a, win, s.d0, s.mhd, st)) return true;
+  // the one-cell kernel: tiles over x and the row axis, z chunks along the
+  // marching axis
+  if (nzc <= 0) nzc = 32;
+  a.nzc = nzc;
   const int kind = fused_kind(nd, s.d0);
   const int tx = kind == 0 ? TileCfg<0>::TX : TileCfg<1>::TX;
   const int ty = kind == 1 ? TileCfg<1>::TY : TileCfg<0>::TY;
@@ -97,12 +105,6 @@ bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win, 
   dim3 grid((s.g.nx[0] + tx - 1) / tx, (s.g.nx[ar] + ty - 1) / ty,
             nd == 3 ? (s.g.nx[am] + nzc - 1) / nzc : 1);
   a.zchunks = grid.z;
-  // 3-D grids: the two-cells-per-thread kernel (packed FP32) where it
-  // applies; VACGPU_PAIR=0 keeps the one-cell kernel
-  if (nd == 3 && launch_sweep_pair(a, s.d0, s.mhd, tmap, nzc, st))
-    return true;
-  // 2-D grids: the warp-marching two-cells-per-thread kernel where it applies
-  if (nd == 2 && launch_sweep_line2(a, win, s.d0, s.mhd, st)) return true;
   const CUtensorMap* map = (const CUtensorMap*)tmap;
   const int D = s.d0;
 #define L1(ND, DD)                                              \

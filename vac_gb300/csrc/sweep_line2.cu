@@ -13,17 +13,18 @@ namespace vacgpu {
 bool pair_enabled();
 bool pair_general(const FusedArgs& a, bool mhd);
 
-// One work item per warp: item = strip + nstrips * chunk.
+// One work item per warp: item = strip + nstrips * chunk of `rows` rows.
 // register bound: four CTAs per SM for HD (128 registers), two for MHD
 template <int D, bool MHD, int LIMC, bool GEN>
 __global__ void __launch_bounds__(L2_NT, MHD ? 2 : 4)
-    k_sweep_line2(const FusedArgs a, const float* __restrict__ win, int nstrips, int nitems) {
+    k_sweep_line2(const FusedArgs a, const float* __restrict__ win, int nstrips, int nitems,
+                  int rows) {
   const int item = blockIdx.x * (L2_NT / 32) + (threadIdx.x >> 5);
   if (item >= nitems) return;
   constexpr int RF = line2_ring_floats(MHD ? 6 : 4);
   __shared__ __align__(16) float ring[L2_NT / 32][RF];
   const int sx = item % nstrips, ch = item / nstrips;
-  const int gya = 2 + ch * L2_ROWS, gyb = min(gya + L2_ROWS, a.g.nx[1] + 2);
+  const int gya = 2 + ch * rows, gyb = min(gya + rows, a.g.nx[1] + 2);
   Line2<D, MHD, LIMC, GEN>::run(a, win, a.wout, ring[threadIdx.x >> 5], sx, gya, gyb,
                                 (unsigned)item);
 }
@@ -68,18 +69,37 @@ bool line2_applies(const FusedArgs& a, bool mhd) {
          a.g.vs * nw < (1LL << 31);
 }
 
-// single-grid work items: strips x chunks of L2_ROWS rows
-static int line2_items(int D, bool mhd, const DevGrid& g, int* nstrips) {
+// Rows per work item of a single grid: the fewest that keep the items within
+// the warps resident at once (four a CTA; two CTAs per SM for MHD, four for
+// HD, 152 SMs), at most L2_ROWS_MAX.  A grid that fits in one wave is bound
+// by the march of one item -- 1.6 us a row, whatever the other warps do --
+// so short items win although each predicts up to three rows beyond its own:
+// a 128^2 MHD sweep takes 12 us in items of 1 row, 64 us in items of 32
+// (512^2: 20 us with 4 rows, 64 with 32; 1001^2: 46 with 16, 64 with 32).
+// Larger grids run several waves: 16 rows took 128 us at 2048^2, 32 rows
+// 130, 8 rows 133.
+constexpr int L2_ROWS_MAX = 16;
+static int line2_rows(int D, bool mhd, const DevGrid& g) {
+  const int strips = line2_strips(D, mhd, g.nx[0]);
+  const int warps = 152 * (mhd ? 2 : 4) * (L2_NT / 32);
+  int rows = 1;
+  while (rows < L2_ROWS_MAX && strips * ((g.nx[1] + rows - 1) / rows) > warps) rows++;
+  return rows;
+}
+
+// single-grid work items: strips x chunks of `rows` rows
+static int line2_items(int D, bool mhd, const DevGrid& g, int rows, int* nstrips) {
   *nstrips = line2_strips(D, mhd, g.nx[0]);
-  return *nstrips * ((g.nx[1] + L2_ROWS - 1) / L2_ROWS);
+  return *nstrips * ((g.nx[1] + rows - 1) / rows);
 }
 
 template <int D, bool MHD, int LIMC, bool GEN>
 static void launch_l2(const FusedArgs& a, const float* win, cudaStream_t st) {
   int ns;
-  const int n = line2_items(D, MHD, a.g, &ns);
+  const int rows = line2_rows(D, MHD, a.g);
+  const int n = line2_items(D, MHD, a.g, rows, &ns);
   const int per = L2_NT / 32;
-  k_sweep_line2<D, MHD, LIMC, GEN><<<(n + per - 1) / per, L2_NT, 0, st>>>(a, win, ns, n);
+  k_sweep_line2<D, MHD, LIMC, GEN><<<(n + per - 1) / per, L2_NT, 0, st>>>(a, win, ns, n, rows);
 }
 
 bool launch_sweep_line2(const FusedArgs& a, const float* win, int D, bool mhd,

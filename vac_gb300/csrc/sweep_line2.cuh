@@ -39,7 +39,6 @@
 namespace vacgpu {
 
 constexpr int L2_NT = 128;   // threads per CTA: four independent warps
-constexpr int L2_ROWS = 32;  // rows per work item
 constexpr int L2_LOOK = 3;   // rows in flight ahead of use
 constexpr int L2_RING = L2_LOOK + 1;  // staging slots per warp
 // a batched work item's strip is bx & L2_STRIP; bit 30 of bx is its sweep

@@ -65,15 +65,37 @@ bool pair_applies(const FusedArgs& a, bool mhd) {
   return a.g.ndim == 3 && !(a.g.xpad & 1) && !(a.g.P & 1);
 }
 
-// False: not applicable, use the one-cell kernel.
-bool launch_sweep_pair(const FusedArgs& a, int D, bool mhd, const void* tmap, int nzc,
+// Planes per CTA (z chunk) of a sweep over `tiles` column tiles and n planes
+// where the caller fixes none: grids of at least three waves (456 CTAs, three
+// per SM, each) in chunks of 32 or 16 planes take those; smaller ones the
+// longest chunk of at most 8 planes that still gives 350 CTAs, down to 2.
+// A CTA marches one plane in 3.7 us alone on its SM and in little more
+// beside two others, so a small grid is bound by the length of the march,
+// although every chunk predicts two planes beyond its own: a 64^3 sweep
+// takes 33 us in chunks of 3 (352 CTAs), 44 in chunks of 8 and 131 in
+// chunks of 32 (32 CTAs); 96^3 65 us with 8, 132 with 32; 127^3 114 with 8,
+// 126 with 16, 164 with 32.
+static int pair_chunk(int tiles, int n) {
+  for (int z : {32, 16})
+    if ((long long)tiles * ((n + z - 1) / z) >= 3 * 456) return z;
+  for (int z : {8, 6, 4, 3})
+    if ((long long)tiles * ((n + z - 1) / z) >= 350) return z;
+  return 2;
+}
+
+// nzc <= 0: pair_chunk's choice.  False: not applicable, use the one-cell
+// kernel.
+bool launch_sweep_pair(FusedArgs a, int D, bool mhd, const void* tmap, int nzc,
                        cudaStream_t st) {
   if (!pair_applies(a, mhd)) return false;
   const int l0 = a.ph.lim[0];
   const int tx = D == 0 ? 30 : 32;
   const int ar = D == 1 ? 2 : 1, am = D == 0 ? 2 : D;
   const int nxt = D == 0 ? (a.g.nx[0] + 1 + tx - 1) / tx : (a.g.nx[0] + tx - 1) / tx;
-  dim3 grid(nxt, (a.g.nx[ar] + 7) / 8, (a.g.nx[am] + nzc - 1) / nzc);
+  const int nyt = (a.g.nx[ar] + 7) / 8;
+  if (nzc <= 0) nzc = pair_chunk(nxt * nyt, a.g.nx[am]);
+  a.nzc = nzc;
+  dim3 grid(nxt, nyt, (a.g.nx[am] + nzc - 1) / nzc);
   const CUtensorMap* map = (const CUtensorMap*)tmap;
 #define LP(DD, M, L) launch_pair_gen<DD, M, L>(map, a, grid, st)
 #define LPD(DD)                                                              \

@@ -199,7 +199,7 @@ struct vacgpu_handle {
   bool fused;
   CUtensorMap tmap[2][2];  // [state buffer][x/z sweeps, y sweep]
   float* idxf[3];
-  int nzc;
+  int nzc;  // planes per CTA (0: the launcher's choice)
   // z-chunk tuning of the fused 3-D sweep (results do not depend on the
   // chunk): pending until the first vacgpu_step call, which times one step
   // per candidate from a snapshot of the state and keeps the fastest
@@ -863,7 +863,7 @@ int vacgpu_internal_view(vacgpu_handle* h, HandleView* v) {
   v->ctrl = h->ctrl;
   for (int i = 0; i < 2; i++)
     for (int k = 0; k < 2; k++) v->tmap[i][k] = &h->tmap[i][k];
-  v->nzc = h->nzc;
+  v->nzc = h->nzc > 0 ? h->nzc : 32;  // a batch fills the GPU with its other grids
   v->fused = h->fused;
   return 0;
 }
@@ -1105,7 +1105,7 @@ int vacgpu_create(const vacgpu_params* p, vacgpu_handle** out) {
     vacgpu_destroy(h);
     return fail(std::string("device allocation failed: ") + cudaGetErrorString(e));
   }
-  h->nzc = 32;
+  h->nzc = 0;  // the launcher's choice, unless pinned or tuned
   if (const char* nz = getenv("VACGPU_NZC")) h->nzc = atoi(nz) > 0 ? atoi(nz) : 32;
   h->fused = p->precision == VACGPU_PREC_MIXED && p->dimsplit &&
              (p->ndim == 2 || p->ndim == 3) && p->ndir == p->ndim &&
@@ -1121,8 +1121,8 @@ int vacgpu_create(const vacgpu_params* p, vacgpu_handle** out) {
         ph.noflux[d][0] || ph.noflux[d][1])
       h->fused = false;
   if (h->fused && p->ndim == 3 && !getenv("VACGPU_NZC") && g.ncell >= (1LL << 21)) {
-    static const int cands[5] = {16, 24, 32, 48, 64};
-    for (int i = 0; i < 5; i++)
+    static const int cands[6] = {8, 16, 24, 32, 48, 64};
+    for (int i = 0; i < 6; i++)
       if (cands[i] < g.nx[2]) h->tcand[h->tncand++] = cands[i];
     h->tuning = h->tncand > 1;
   }

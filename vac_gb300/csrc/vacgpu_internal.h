@@ -280,7 +280,7 @@ void launch_correct_roe_mixed(const SweepArgs& s, const float* w,
 // Fused single-kernel sweep of the mixed path (sweep_fused.cu): returns
 // false when no fused instance exists for the configuration.  `tmap` is the
 // CUtensorMap (as bytes) of the input state buffer with the box of the sweep
-// direction (fused_box_rows).
+// direction (fused_box_rows); nzc: planes per CTA (0: chosen by size).
 bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win,
                         float* wout,
                         const float* const* idxf, int nzc, cudaStream_t st);
