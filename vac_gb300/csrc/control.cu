@@ -18,6 +18,53 @@ __global__ void k_smallp(Ctrl* c, int mhd, double coeff) {
 }
 __global__ void k_dt_end(Ctrl* c, DtEndArgs p) { dt_end_dev(c, p); }
 __global__ void k_step_end(Ctrl* c, int ndim) { step_end_dev(c, ndim, 0); }
+// A shared-memory copy of the control block's scalars: one trip to L2 for
+// all of them, instead of one for each field that a thread reads.
+struct HeadCopy {
+  static constexpr int N = sizeof(CtrlHead) / 8;
+  static_assert(N <= NSLOT, "one word per thread");
+  static __device__ __forceinline__ void get(CtrlHead* s, const CtrlHead* c) {
+    if ((int)threadIdx.x < N)
+      ((unsigned long long*)s)[threadIdx.x] = ((const unsigned long long*)c)[threadIdx.x];
+    __syncthreads();
+  }
+  static __device__ __forceinline__ void put(const CtrlHead* s, CtrlHead* c) {
+    __syncthreads();
+    if ((int)threadIdx.x < N)
+      ((unsigned long long*)c)[threadIdx.x] = ((const unsigned long long*)s)[threadIdx.x];
+  }
+};
+
+// The end of a step and the dt choice of the next one in one launch.  The
+// time loop between two sweeps was six (step_end, dt_begin, the first-step
+// passes and smallp, which do nothing after the first step, dt_end).
+__global__ void __launch_bounds__(NSLOT) k_step_ctl(Ctrl* c, int ndim, DtEndArgs p) {
+  __shared__ CtrlHead s;
+  HeadCopy::get(&s, c);
+  if (s.done) return;
+  step_end_dev(&s, c, ndim, 0);
+  __syncthreads();
+  choose_dt_dev(&s, c, ndim, p);
+  HeadCopy::put(&s, c);
+}
+// The start of a call, with the dt choice of its first step unless the host
+// issues that step's passes itself (choose = 0).
+__global__ void __launch_bounds__(NSLOT)
+    k_call_ctl(Ctrl* c, int ndim, DtEndArgs p, int maxsteps, double tstop, int choose) {
+  __shared__ CtrlHead s;
+  HeadCopy::get(&s, c);
+  if (threadIdx.x == 0) {
+    s.done = 0;
+    s.steps = 0;
+    s.maxsteps = maxsteps;
+    s.tstop = tstop;
+  }
+  __syncthreads();
+  if (choose) choose_dt_dev(&s, c, ndim, p);
+  HeadCopy::put(&s, c);
+}
+// after done = 4: the host issues the passes of the pending step
+__global__ void k_resume(Ctrl* c) { c->done = 0; }
 
 // batched: block b serves grid b
 __global__ void kb_dt_begin(Ctrl* const* cs, int ndim) {
@@ -180,6 +227,14 @@ void launch_dt_end(Ctrl* c, const vacgpu_params& p, cudaStream_t st) {
 void launch_step_end(Ctrl* c, int ndim, cudaStream_t st) {
   k_step_end<<<1, NSLOT, 0, st>>>(c, ndim);
 }
+void launch_step_ctl(Ctrl* c, const vacgpu_params& p, cudaStream_t st) {
+  k_step_ctl<<<1, NSLOT, 0, st>>>(c, p.ndim, dt_end_args(p));
+}
+void launch_call_ctl(Ctrl* c, const vacgpu_params& p, int maxsteps, double tstop, int choose,
+                     cudaStream_t st) {
+  k_call_ctl<<<1, NSLOT, 0, st>>>(c, p.ndim, dt_end_args(p), maxsteps, tstop, choose);
+}
+void launch_resume(Ctrl* c, cudaStream_t st) { k_resume<<<1, 1, 0, st>>>(c); }
 
 void launchb_control(int which, Ctrl* const* cs, int n, const vacgpu_params& p,
                      int toggle, int maxsteps, double tstop, cudaStream_t st) {

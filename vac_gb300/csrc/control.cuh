@@ -34,7 +34,9 @@ __device__ __forceinline__ unsigned long long fold_max(const unsigned long long*
   return r;
 }
 
-__device__ __forceinline__ void dt_begin_dev(Ctrl* c, int ndim) {
+// (the control functions take the scalars h and the slot arrays of a control
+// block apart: k_step_ctl works on a shared-memory copy of the scalars)
+__device__ __forceinline__ void dt_begin_dev(CtrlHead* c, Ctrl* k, int ndim) {
   __shared__ int stop;
   if (threadIdx.x == 0) {
     stop = c->done;
@@ -56,13 +58,14 @@ __device__ __forceinline__ void dt_begin_dev(Ctrl* c, int ndim) {
   if (stop) return;
   const int i = threadIdx.x;
   for (int d = 0; d < 3; d++) {
-    c->face_cmax[d][i] = 0ULL;
-    c->face_cmax2[d][i] = 0ULL;
-    c->cell_cmax[d][i] = 0ULL;
+    k->face_cmax[d][i] = 0ULL;
+    k->face_cmax2[d][i] = 0ULL;
+    k->cell_cmax[d][i] = 0ULL;
   }
-  c->pmin[i] = ~0ULL;
-  c->pmax[i] = 0ULL;
+  k->pmin[i] = ~0ULL;
+  k->pmax[i] = 0ULL;
 }
+__device__ __forceinline__ void dt_begin_dev(Ctrl* c, int ndim) { dt_begin_dev(c, c, ndim); }
 
 // smallp = minval(p)*smallpcoeff at the first getpthermal call; MHD falls
 // back to maxval(p)*smallpcoeff for a negative minimum
@@ -96,11 +99,11 @@ struct DtEndArgs {
 };
 DtEndArgs dt_end_args(const vacgpu_params& p);  // control.cu
 
-__device__ __forceinline__ void dt_end_dev(Ctrl* c, const DtEndArgs& p) {
+__device__ __forceinline__ void dt_end_dev(CtrlHead* c, const Ctrl* k, const DtEndArgs& p) {
   if (c->done) return;
   unsigned long long km[3] = {0, 0, 0};
   for (int d = 0; d < p.ndim; d++)
-    if (c->need_cell[d]) km[d] = fold_max(c->cell_cmax[d]);
+    if (c->need_cell[d]) km[d] = fold_max(k->cell_cmax[d]);
   if (threadIdx.x != 0) return;
   double dt;
   double dtc_save[3] = {c->dtcourant[0], c->dtcourant[1], c->dtcourant[2]};
@@ -173,19 +176,50 @@ __device__ __forceinline__ void dt_end_dev(Ctrl* c, const DtEndArgs& p) {
   }
   c->dt = dt;
 }
+__device__ __forceinline__ void dt_end_dev(Ctrl* c, const DtEndArgs& p) { dt_end_dev(c, c, p); }
 
 // After the last sweep: fold the correctors' CFL maxima into dtcourant
 // (src/vactvdlf.t:184-201; 'tvdmu': the fast waves' normalised
 // eigenvalues, src/vactvd.t:144-160), count Courant violations, it+1, t+dt.
 // toggle: the number of buffer swaps of one step (batched grids).
-__device__ __forceinline__ void step_end_dev(Ctrl* c, int ndim, int toggle) {
-  if (c->done) return;
-  unsigned long long km[3] = {0, 0, 0}, km2[3] = {0, 0, 0};
-  if (c->courantpar > 0.0)
-    for (int d = 0; d < ndim; d++) {
-      km[d] = fold_max(c->face_cmax[d]);
-      if (c->roe) km2[d] = fold_max(c->face_cmax2[d]);
+//
+// The maxima of the slots (face_cmax of d < ndim, then face_cmax2), in every
+// thread: the loads of all arrays are in flight together and the lanes fold
+// by shuffles, one barrier pair in all.
+__device__ __forceinline__ void fold_faces(const Ctrl* k, int ndim, int roe,
+                                           unsigned long long* km) {
+  __shared__ unsigned long long sh[6][NSLOT / 32];
+  unsigned long long v[6];
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    const unsigned long long* s = i < 3 ? k->face_cmax[i] : k->face_cmax2[i - 3];
+    v[i] = (i % 3 < ndim && (i < 3 || roe)) ? __ldcg(s + threadIdx.x) : 0ULL;
+  }
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    if (!(i % 3 < ndim && (i < 3 || roe))) continue;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long u = __shfl_xor_sync(0xffffffffu, v[i], o);
+      v[i] = u > v[i] ? u : v[i];
     }
+    if ((threadIdx.x & 31) == 0) sh[i][threadIdx.x >> 5] = v[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    km[i] = 0ULL;
+    if (!(i % 3 < ndim && (i < 3 || roe))) continue;
+#pragma unroll
+    for (int w = 0; w < NSLOT / 32; w++) km[i] = sh[i][w] > km[i] ? sh[i][w] : km[i];
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void step_end_dev(CtrlHead* c, const Ctrl* k, int ndim, int toggle) {
+  if (c->done) return;
+  unsigned long long km[6] = {0, 0, 0, 0, 0, 0};
+  if (c->courantpar > 0.0) fold_faces(k, ndim, c->roe, km);
+  const unsigned long long* km2 = km + 3;
   if (threadIdx.x != 0) return;
   for (int d = 0; d < ndim; d++) {
     if (c->roe) {
@@ -215,6 +249,27 @@ __device__ __forceinline__ void step_end_dev(Ctrl* c, int ndim, int toggle) {
   c->t = c->t + c->dt;
   c->steps = c->steps + 1;
   c->cur ^= toggle;
+}
+__device__ __forceinline__ void step_end_dev(Ctrl* c, int ndim, int toggle) {
+  step_end_dev(c, c, ndim, toggle);
+}
+
+// The dt choice of the next step where it needs no pass over the grid
+// (dt_begin, then dt_end).  A step that does need the cell-centred passes
+// (its dtcourant is unset: a first step, or wave speeds that gave none) is
+// left to the host: done = 4 stops the kernels issued after it until the
+// host has run those passes (resume_dt in vacgpu.cu).
+__device__ __forceinline__ void choose_dt_dev(CtrlHead* c, Ctrl* k, int ndim,
+                                              const DtEndArgs& p) {
+  __shared__ int need;
+  dt_begin_dev(c, k, ndim);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    need = !c->done && (c->need_smallp | c->need_cell[0] | c->need_cell[1] | c->need_cell[2]);
+    if (need) c->done = 4;
+  }
+  __syncthreads();
+  if (!need) dt_end_dev(c, k, p);
 }
 
 }  // namespace vacgpu

@@ -28,6 +28,7 @@
 
 int vacgpu_internal_fail(const char* msg);
 int vacgpu_internal_step_async(vacgpu_handle* h, int k);
+int vacgpu_internal_steps_left(vacgpu_handle* h, int* left);
 void* vacgpu_internal_stream(vacgpu_handle* h);
 size_t vacgpu_internal_device_bytes(const vacgpu_params* p);
 
@@ -173,9 +174,15 @@ void worker_loop(vacgpu_server* s) {
         continue;
       }
       progressed = true;
-      if (r->issued < r->nsteps) {
+      bool ok = true;
+      if (r->issued == r->nsteps) {
+        int left = 0;  // steps that wait for the first-step passes
+        ok = vacgpu_internal_steps_left(r->h, &left) == 0;
+        r->issued -= left;
+      }
+      if (!ok || r->issued < r->nsteps) {
         const int k = r->nsteps - r->issued < s->chunk ? r->nsteps - r->issued : s->chunk;
-        if (vacgpu_internal_step_async(r->h, k) ||
+        if (!ok || vacgpu_internal_step_async(r->h, k) ||
             cudaEventRecord(r->ev, (cudaStream_t)vacgpu_internal_stream(r->h)) !=
                 cudaSuccess) {
           char buf[512];

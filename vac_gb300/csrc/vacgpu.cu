@@ -109,13 +109,6 @@ __global__ void k_sums_final(const double* part, long long nblk, int nw,
   out[iw] = s;
 }
 
-__global__ void k_call_begin(Ctrl* c, int maxsteps, double tstop) {
-  c->done = 0;
-  c->steps = 0;
-  c->maxsteps = maxsteps;
-  c->tstop = tstop;
-}
-
 }  // namespace
 
 int vacgpu_internal_fail(const char* msg) { return fail(msg); }
@@ -163,6 +156,12 @@ struct vacgpu_handle {
   unsigned special[VACGPU_MAXB];  // per region: bit iw 'special'
   double* xg[3];     // cell centres over the ghost box (specialbound hooks)
   int cur;           // which of buf[0], buf[1] holds the state
+  bool fresh;        // no step has run since the upload
+  int async_cur, async_it;  // cur and it when step_async last began fresh
+  // done and steps of the control block after each of the two chunks of
+  // steps in flight (page-locked), and the events behind those copies
+  int* poll;
+  cudaEvent_t poll_ev[2];
   double* dx[3];
   float* dxf[3];
   std::vector<double> hdx[3];
@@ -605,8 +604,16 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
   h->cur ^= 1;
 }
 
+// Every step chooses its dt with the passes of run_dt and ends with
+// launch_step_end where a user hook or the specialeta field takes part in
+// the choice; elsewhere launch_step_ctl ends a step and chooses the next
+// one's dt, and run_dt serves the first step after an upload.
+bool dt_each_step(const vacgpu_handle* h) { return h->dtsp_fn || h->etaf; }
+
+// The dt choice with the first-step passes (each does nothing unless this
+// step needs it).
 template <typename T>
-void run_step(vacgpu_handle* h, int parity_odd) {
+void run_dt(vacgpu_handle* h) {
   const vacgpu_params& p = h->p;
   SweepArgs a = make_args(h, 0, p.ndim - 1);
   kbegin(h, VACGPU_K_CONTROL);
@@ -651,6 +658,15 @@ void run_step(vacgpu_handle* h, int parity_odd) {
   kbegin(h, VACGPU_K_CONTROL);
   launch_dt_end(h->ctrl, p, h->st);
   kend(h);
+}
+
+// One step: with the general dt choice before it, or (ctl) its end and the
+// dt choice of the next step after it.
+template <typename T>
+void run_step(vacgpu_handle* h, int parity_odd) {
+  const vacgpu_params& p = h->p;
+  const bool each = dt_each_step(h);
+  if (each) run_dt<T>(h);
   if (p.typelimited == VACGPU_LIMITED_PREVIOUS && p.dimsplit)
     cudaMemcpyAsync(h->wold, h->buf[h->cur], h->elem * h->g.vs * h->nw,
                     cudaMemcpyDeviceToDevice, h->st);
@@ -664,8 +680,40 @@ void run_step(vacgpu_handle* h, int parity_odd) {
     run_sweep<T>(h, 0, p.ndim - 1);
   }
   kbegin(h, VACGPU_K_CONTROL);
-  launch_step_end(h->ctrl, p.ndim, h->st);
+  if (each)
+    launch_step_end(h->ctrl, p.ndim, h->st);
+  else
+    launch_step_ctl(h->ctrl, p, h->st);
   kend(h);
+}
+
+void run_dt_any(vacgpu_handle* h) {
+  if (h->elem == 8)
+    run_dt<double>(h);
+  else
+    run_dt<float>(h);
+}
+
+// The start of a call of up to maxsteps steps: with run_dt where no step
+// has run since the upload (fresh), else with the dt choice in the launch.
+void begin_call(vacgpu_handle* h, int maxsteps, double tstop) {
+  const bool each = dt_each_step(h);
+  kbegin(h, VACGPU_K_CONTROL);
+  launch_call_ctl(h->ctrl, h->p, maxsteps, tstop, !each && !h->fresh, h->st);
+  kend(h);
+  if (!each && h->fresh && maxsteps > 0) {
+    run_dt_any(h);
+    h->fresh = false;
+  }
+}
+
+// After done = 4 with `steps` steps done of those issued from buffer cur0:
+// the passes of the pending step's dt choice.
+void resume_dt(vacgpu_handle* h, int cur0, int steps) {
+  const int nsw = h->p.dimsplit ? h->p.ndim : 1;
+  h->cur = cur0 ^ ((steps * nsw) & 1);
+  launch_resume(h->ctrl, h->st);
+  run_dt_any(h);
 }
 
 // Issue k steps on the handle's stream without waiting: two-step units
@@ -692,7 +740,8 @@ int tune_nzc(vacgpu_handle* h) {
   int nbest = h->nzc;
   for (int i = 0; i < h->tncand; i++) {
     h->nzc = h->tcand[i];
-    k_call_begin<<<1, 1, 0, h->st>>>(h->ctrl, 1, 1e300);
+    launch_call_ctl(h->ctrl, h->p, 1, 1e300, 0, h->st);
+    if (!dt_each_step(h)) run_dt<float>(h);
     cudaEventRecord(e0, h->st);
     run_step<float>(h, h->it_host & 1);
     cudaEventRecord(e1, h->st);
@@ -876,10 +925,29 @@ int vacgpu_internal_set_cur(vacgpu_handle* h, int cur) {
 // between) without any host synchronisation.
 int vacgpu_internal_step_async(vacgpu_handle* h, int k) {
   h->tuning = false;  // served solves keep the default z chunk
-  k_call_begin<<<1, 1, 0, h->st>>>(h->ctrl, k, 1e300);
+  if (h->fresh) {
+    h->async_cur = h->cur;
+    h->async_it = h->it_host;
+  }
+  begin_call(h, k, 1e300);
   if (issue_steps(h, k, h->it_host)) return 1;
   h->it_host += k;
   CK(cudaGetLastError());
+  return 0;
+}
+// After the steps of vacgpu_internal_step_async ran: how many of those
+// issued are still to do, because a step waits for the first-step passes
+// (every later call stops there as well; the next one issues the passes).
+// None are where not one ran since those passes: the run is finished.
+int vacgpu_internal_steps_left(vacgpu_handle* h, int* left) {
+  int st[3];  // it, itmin, done
+  CK(cudaMemcpyAsync(st, &h->ctrl->it, sizeof(st), cudaMemcpyDeviceToHost, h->st));
+  CK(cudaStreamSynchronize(h->st));
+  *left = st[2] == 4 && st[0] != h->async_it ? h->it_host - st[0] : 0;
+  h->it_host = st[0];
+  const int nsw = h->p.dimsplit ? h->p.ndim : 1;
+  h->cur = h->async_cur ^ (((st[0] - h->async_it) * nsw) & 1);
+  if (st[2] == 4) h->fresh = true;
   return 0;
 }
 void* vacgpu_internal_stream(vacgpu_handle* h) { return (void*)h->st; }
@@ -1310,6 +1378,7 @@ int vacgpu_upload(vacgpu_handle* h, const double* w, int it, double t) {
   CK(cudaStreamSynchronize(h->st));
   if (h->hook_failed) return fail("the specialbound hook failed");
   h->cur = 0;
+  h->fresh = true;
   h->it_host = it;
   h->have_state = true;
   return 0;
@@ -1390,6 +1459,9 @@ const double* vacgpu_snapshot_data(vacgpu_handle* h, int slot) {
   return sn.host;
 }
 
+// steps issued between two reads of the done flag
+static constexpr int STEP_CHUNK = 8;
+
 int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
                 int* it, double* dt, int* finished) {
   if (!h) return fail("null handle");
@@ -1403,32 +1475,52 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
   if (h->tuning && maxsteps > 0 && !h->timing && tune_nzc(h)) return 1;
   const int nsw = h->p.dimsplit ? h->p.ndim : 1;
   const int start_cur = h->cur;
-  kbegin(h, VACGPU_K_CONTROL);
-  k_call_begin<<<1, 1, 0, h->st>>>(h->ctrl, maxsteps, tstop);
-  kend(h);
+  begin_call(h, maxsteps, tstop);
   CK(cudaGetLastError());
-  int issued = 0, chunk = 4;
+  // Steps are issued in chunks, two in flight, so the device does not wait
+  // for the host between chunks; each chunk's done flag is read back behind
+  // it, and no more are issued once one reports a stop.
+  int issued = 0, head = 0, inflight = 0, chunk = STEP_CHUNK;
   Ctrl c;
-  while (issued < maxsteps) {
-    int k = maxsteps - issued < chunk ? maxsteps - issued : chunk;
-    if (issue_steps(h, k, h->it_host + issued)) return 1;
-    issued += k;
-    CK(cudaGetLastError());
-    if (h->hook_failed) {
-      h->hook_failed = false;
-      drop_graphs(h);
-      CK(cudaStreamSynchronize(h->st));
-      return fail("a user hook (specialbound, specialeta, specialsource or getdt_special) failed");
+  while (true) {
+    bool stop = false;
+    while (issued < maxsteps && !stop) {
+      const int k = maxsteps - issued < chunk ? maxsteps - issued : chunk;
+      if (issue_steps(h, k, h->it_host + issued)) return 1;
+      issued += k;
+      CK(cudaGetLastError());
+      if (h->hook_failed) {
+        h->hook_failed = false;
+        drop_graphs(h);
+        CK(cudaStreamSynchronize(h->st));
+        return fail("a user hook (specialbound, specialeta, specialsource or getdt_special) failed");
+      }
+      if (issued == maxsteps) break;  // the control block is read below
+      if (!h->poll) {
+        for (cudaEvent_t& e : h->poll_ev)
+          if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        CK(cudaMallocHost(&h->poll, 4 * sizeof(int)));
+      }
+      const int slot = (head + inflight) & 1;
+      CK(cudaMemcpyAsync(h->poll + 2 * slot, &h->ctrl->done, 2 * sizeof(int),
+                         cudaMemcpyDeviceToHost, h->st));
+      CK(cudaEventRecord(h->poll_ev[slot], h->st));
+      if (++inflight < 2) continue;
+      CK(cudaEventSynchronize(h->poll_ev[head]));
+      stop = h->poll[2 * head] != 0;
+      head ^= 1;
+      inflight--;
     }
-    int done = 0;
-    CK(cudaMemcpyAsync(&done, &h->ctrl->done, sizeof(int),
-                       cudaMemcpyDeviceToHost, h->st));
+    CK(cudaMemcpyAsync(&c, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
-    if (done) break;
-    if (chunk < 64) chunk *= 2;
+    inflight = 0;
+    if (c.done != 4) break;
+    // a step later than the first needs the first-step passes: run them,
+    // and go on from the steps done, one at a time
+    resume_dt(h, start_cur, c.steps);
+    issued = c.steps;
+    chunk = 1;
   }
-  CK(cudaMemcpyAsync(&c, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
   // every executed step swapped the buffers nsw times; skipped ones none
   h->cur = start_cur ^ ((c.steps * nsw) & 1);
   if (c.fault) {
@@ -1581,6 +1673,9 @@ void vacgpu_destroy(vacgpu_handle* h) {
   cudaFree(h->part);
   cudaFree(h->sums);
   cudaFree(h->ctrl);
+  cudaFreeHost(h->poll);
+  for (cudaEvent_t e : h->poll_ev)
+    if (e) cudaEventDestroy(e);
   drain_events(h);
   for (auto e : h->pool) cudaEventDestroy(e);
   for (int i = 0; i < 2; i++)

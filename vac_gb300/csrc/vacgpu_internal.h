@@ -123,7 +123,7 @@ __host__ __device__ inline int gmap_src(int gi, int n, int m) {
 // Device-resident time-loop state: dt, it and t never leave the device
 // between steps, so a sequence of steps runs without host round trips (and
 // can be captured as one CUDA graph).
-struct Ctrl {
+struct CtrlHead {
   double t, dt, dtold, dtpar, courantpar;
   double smallp;
   double dtgrav;
@@ -137,23 +137,29 @@ struct Ctrl {
   double tstop;
   double dtcourant[3];
   int it, itmin;
-  int done;           // 0 running, 1 timetofinish, 2 tstop, 3 maxsteps
-  int steps;          // steps done in the current vacgpu_step call
+  // 0 running, 1 timetofinish, 2 tstop, 3 maxsteps, 4 the next step waits
+  // for the first-step passes (choose_dt_dev)
+  int done;
+  int steps;          // steps done in the current vacgpu_step call (after done)
   int maxsteps;
   int need_cell[3];   // this step's dt needs the cell-centred cmax pass
   int need_smallp;    // smallp<0 at this step's first pressure evaluation
   int nerror[4];
   int fault;          // a bounded device wait gave up (TMA never completed)
+  int roe;            // 'tvdmu': two fast-wave maxima per direction
   int cur;            // batched grids: which state buffer holds the state
   double smallrho;    // keeppositive_rho: -1 until set from min(rho)
   int need_smallrho;  // this keeppositive call sets smallrho
   int kp_r, kp_p;     // this keeppositive call found small rho / p
+};
+static_assert(sizeof(CtrlHead) % 8 == 0, "copied as 8-byte words");
+
+struct Ctrl : CtrlHead {
   // grid-level reductions (ordered-integer keys, atomicMax/atomicMin)
   unsigned long long face_cmax[3][NSLOT];  // corrector max cmax*2/(dx+dx)
   // 'tvdmu': max |a|*dt*2/(dx+dx) of the fastRW (face_cmax) and fastLW
   // (face_cmax2) waves of tvdlimit2 (src/vactvd.t:144-160)
   unsigned long long face_cmax2[3][NSLOT];
-  int roe;
   unsigned long long cell_cmax[3][NSLOT];  // getdt_courant max cmax/dx
   unsigned long long pmin[NSLOT], pmax[NSLOT];
   unsigned long long rmin[NSLOT];          // keeppositive_rho min(rho)
@@ -308,6 +314,13 @@ void launch_set_qt(Ctrl* c, int mode, cudaStream_t st);
 // specialeta: Ctrl::etak from the field (first_only: at it==itmin only)
 void launch_eta_max(const SweepArgs& a, int first_only, cudaStream_t st);
 void launch_step_end(Ctrl* c, int ndim, cudaStream_t st);
+// step_end and the dt choice of the next step; the start of a call (choose:
+// with the dt choice of its first step); both leave done = 4 where the next
+// step needs the first-step passes, which launch_resume clears
+void launch_step_ctl(Ctrl* c, const vacgpu_params& p, cudaStream_t st);
+void launch_call_ctl(Ctrl* c, const vacgpu_params& p, int maxsteps, double tstop, int choose,
+                     cudaStream_t st);
+void launch_resume(Ctrl* c, cudaStream_t st);
 // Batched control: which = 0 dt_begin, 1 smallp, 2 dt_end, 3 step_end
 // (toggle = buffer swaps per step), 4 call_begin; one block per grid.
 void launchb_control(int which, Ctrl* const* cs, int n, const vacgpu_params& p,
