@@ -515,3 +515,26 @@ def test_isentropic_vortex_one_crossing(gpu_lib, precision):
             rel = np.abs(got[iw] - ref[iw]).sum() / np.abs(ref[iw]).sum()
             assert rel <= MIXED_REL_L1, (iw, rel)
     assert np.abs(got[0] - s.w[0]).mean() < (1.2e-2 if n == 32 else 3e-3)
+
+
+@pytest.mark.parametrize("lim", ["minmod", "woodward", "superbee", "vanleer"])
+@pytest.mark.parametrize("ndim", [1, 2, 3])
+def test_fp64_slopes_of_zeros_and_ties(gpu_lib, lim, ndim):
+    """States full of exact zeros (of either sign), equal neighbours and sign
+    changes, where a limiter's comparisons tie: bit for bit the oracle's."""
+    rng = np.random.default_rng(17 + ndim)
+    nx = {1: (301,), 2: (23, 31), 3: (13, 9, 11)}[ndim]
+    x = inistate.domain_grid(nx, (0.0,) * ndim, (1.0,) * ndim)
+    rho = rng.choice([1.0, 1.0, 1.25, 1.5], size=nx)
+    mom = [rng.choice([0.0, -0.0, 0.0, 0.25, -0.25, 0.125], size=nx) for _ in range(ndim)]
+    b = [rng.choice([0.0, -0.0, 0.5, 0.5, -0.5], size=nx) for _ in range(ndim)] if ndim > 1 else []
+    e = 4.0 + sum(m * m for m in mom) + sum(q * q for q in b)
+    s = inistate.sod_1d(8)
+    s.header = "ties" + ("_mhd%d%d" % (ndim, ndim) if b else "_hd%d%d" % (ndim, ndim))
+    s.ndim, s.nx, s.x, s.w = ndim, nx, x, np.stack([rho] + mom + [e] + b)
+    p = inistate.params_for(s, limiter=lim, bc="periodic" if ndim == 2 else "cont")
+    g, o = Engine(p, s.x, s.w), Oracle(p, s.x, s.w)
+    g.step(3)
+    o.step(3)
+    assert g.t == o.t
+    assert np.array_equal(g.state().view(np.uint64), o.state().view(np.uint64))

@@ -212,6 +212,8 @@ DtEndArgs dt_end_args(const vacgpu_params& p) {
   a.etafield = p.physics == VACGPU_PHYS_MHD && p.eqpar[1] < 0.0;
   a.dtdiffpar = p.dtdiffpar;
   a.ndim = p.ndim;
+  a.fp64 = p.precision == VACGPU_PREC_FP64;
+  a.nsweep = p.dimsplit ? 1 : p.ndim;
   a.itmax = p.itmax;
   a.slowsteps = p.slowsteps;
   a.dtcantgrow = p.dtcantgrow;

@@ -92,7 +92,9 @@ __device__ __forceinline__ void smallp_dev(Ctrl* c, int mhd, double coeff) {
 }
 
 struct DtEndArgs {
-  int ndim, itmax, slowsteps, dtcantgrow, tmaxexact;
+  int ndim, nsweep;   // nsweep: directions a source call covers (split: 1)
+  int fp64;           // the FP64 path reads CtrlHead::srcq
+  int itmax, slowsteps, dtcantgrow, tmaxexact;
   double tmax, dtmin;
   int etafield;       // specialeta: dtdiff from the field's max eta/dx^2
   double dtdiffpar;
@@ -175,6 +177,12 @@ __device__ __forceinline__ void dt_end_dev(CtrlHead* c, const Ctrl* k, const DtE
     if (q < dt) dt = q;
   }
   c->dt = dt;
+  if (p.fp64) {
+    // qdt*nsweep/ndim; the predictor's is half the corrector's, exactly
+    const double q = dt * (double)p.nsweep;
+    c->srcq[1] = p.ndim == 1 ? q : p.ndim == 2 ? 0.5 * q : q / 3.0;
+    c->srcq[0] = 0.5 * c->srcq[1];
+  }
 }
 __device__ __forceinline__ void dt_end_dev(Ctrl* c, const DtEndArgs& p) { dt_end_dev(c, c, p); }
 

@@ -34,10 +34,12 @@ std::mutex g_mu;
 
 // Every call starts from a clean control block: the scratch keeps the last
 // call's contents, so the CFL slots must be zeroed and done cleared.
-__global__ void k_na_begin(Ctrl* c, double dt, double smallp) {
+__global__ void k_na_begin(Ctrl* c, double dt, double smallp, int ndim) {
   if (threadIdx.x == 0) {
     c->done = 0;
     c->dt = dt;
+    c->srcq[0] = dt / 2 * 1.0 / ndim;
+    c->srcq[1] = dt * 1.0 / ndim;
     c->smallp = smallp;
   }
   for (int d = 0; d < 3; d++) c->face_cmax[d][threadIdx.x] = 0ULL;
@@ -179,7 +181,7 @@ extern "C" int vacgpu_sweep_noalloc(const vacgpu_params* p, const double* w,
   s.face_stride = (long long)p->nw * face_count(g, idim);
 
   cudaStream_t st = (cudaStream_t)stream;
-  k_na_begin<<<1, NSLOT, 0, st>>>(a.ctrl, dt, p->smallp);
+  k_na_begin<<<1, NSLOT, 0, st>>>(a.ctrl, dt, p->smallp, p->ndim);
   if (p->typefull == VACGPU_TVDLF1) {
     // onestep (typepred1='nul'): the corrector alone with wCT = w and no
     // limiter (src/vacio.t:286-299,511)

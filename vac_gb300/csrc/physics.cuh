@@ -4,7 +4,11 @@
 // The FP64 functions keep every Fortran array statement of the reference as
 // the same sequence of IEEE operations (this header is compiled without FMA
 // contraction for the FP64 path), so each value is bit-identical to the CPU
-// restatement.  Variable layout (src/vacpar.t.mhd:9-26, src/vacpar.t.hd:9-26):
+// restatement.  A factor that is a power of two is folded into an FMA where
+// the reference multiplies by it and adds: the product is exact, so the
+// FMA rounds once, where the reference's sum does (every result above the
+// subnormal range keeps its bits, and the FP64 pipe, which bounds these
+// kernels, issues one operation less).  Variable layout (src/vacpar.t.mhd:9-26, src/vacpar.t.hd:9-26):
 //   rho=0, m_c=c (c=1..NDIR), e=NDIR+1, b_c=NDIR+1+c.
 #pragma once
 #include <cuda_runtime.h>
@@ -30,9 +34,46 @@ typedef DevPhys PhysConst;
 
 // ------------------------------------------------------------------ FP64
 
+// Several IEEE quotients by one denominator.  A state is divided by its
+// density five times in a flux, and CUDA's division costs nine operations of
+// the FP64 pipe each time; here the reciprocal is formed once and a quotient
+// takes four: with y = RN(1/b) and yl = 1/b - y to a few bits,
+// q = RN(a*y + RN(a*yl)) is within an ulp of a/b, its remainder r = a - b*q
+// is exact, and RN(q + r*y) is then a/b correctly rounded (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34 (1990), theorem on quotients).  That holds
+// away from overflow and underflow: b in [2^-100, 2^100] and |a| in
+// [2^-800, 2^800], tested on the exponents.  A zero a over such a b is the
+// quotient itself -- gas at rest or unmagnetised has one in most divisions,
+// and CUDA's division leaves its fast path for it; everything else takes
+// CUDA's division.
+static __device__ __noinline__ double div_any(double a, double b) { return a / b; }
+struct Rcp64 {
+  double b, y, yl;
+  bool ok;
+};
+__device__ __forceinline__ bool exponent_within(double x, unsigned e) {
+  return (((unsigned)__double2hiint(x) >> 20 & 0x7ffu) - (1023u - e)) <= 2u * e;
+}
+__device__ __forceinline__ Rcp64 rcp64(double b) {
+  Rcp64 r;
+  r.b = b;
+  r.y = __drcp_rn(b);
+  r.yl = fma(-b, r.y, 1.0) * r.y;
+  r.ok = __double2hiint(b) > 0 && exponent_within(b, 100);
+  return r;
+}
+__device__ __forceinline__ double div64(double a, const Rcp64& r) {
+  double q = fma(a, r.y, a * r.yl);
+  q = fma(fma(-r.b, q, a), r.y, q);
+  if (!(r.ok && exponent_within(a, 800)))
+    q = r.ok && (__double_as_longlong(a) << 1) == 0 ? a : div_any(a, r.b);
+  return q;
+}
+
 // getptotal, src/vacphys0.t.mhd:225-257 (unclipped total pressure)
 template <int NDIR>
-__device__ __forceinline__ double ptotal_mhd(const double* u,
+__device__ __forceinline__ double ptotal_mhd(const double* u, const Rcp64& ir,
                                              const PhysConst& k) {
   typedef Lay<NDIR, true> L;
   double bb = u[L::B0 + 1] * u[L::B0 + 1];
@@ -43,33 +84,34 @@ __device__ __forceinline__ double ptotal_mhd(const double* u,
   double mm = u[1] * u[1];
 #pragma unroll
   for (int c = 2; c <= NDIR; c++) mm = mm + u[c] * u[c];
-  p = p - k.pt3 * mm / u[0];
+  p = p - div64(k.pt3 * mm, ir);
   return p;
 }
 
 // getpthermal, src/vacphys0.t.mhd:165-222 (before clipping)
+// (ir: u[0] and its reciprocal)
 template <int NDIR>
-__device__ __forceinline__ double pthermal_mhd_raw(const double* u,
+__device__ __forceinline__ double pthermal_mhd_raw(const double* u, const Rcp64& ir,
                                                    const PhysConst& k) {
   typedef Lay<NDIR, true> L;
   double mm = u[1] * u[1];
 #pragma unroll
   for (int c = 2; c <= NDIR; c++) mm = mm + u[c] * u[c];
-  double p = mm / u[0];
+  double p = div64(mm, ir);
 #pragma unroll
   for (int c = 1; c <= NDIR; c++) p = p + u[L::B0 + c] * u[L::B0 + c];
-  return k.gm1 * (u[L::E] - 0.5 * p);
+  return k.gm1 * fma(-0.5, p, u[L::E]);  // e - 0.5*p
 }
 
 // getpthermal, src/vacphys0.t.hd:103-134 (before clipping)
 template <int NDIR>
-__device__ __forceinline__ double pthermal_hd_raw(const double* u,
+__device__ __forceinline__ double pthermal_hd_raw(const double* u, const Rcp64& ir,
                                                   const PhysConst& k) {
   typedef Lay<NDIR, false> L;
   double mm = u[1] * u[1];
 #pragma unroll
   for (int c = 2; c <= NDIR; c++) mm = mm + u[c] * u[c];
-  return k.gm1 * (u[L::E] - 0.5 * mm / u[0]);
+  return k.gm1 * fma(-0.5, div64(mm, ir), u[L::E]);  // e - 0.5*mm/rho
 }
 
 __device__ __forceinline__ double clip_p(double p, double smallp) {
@@ -79,8 +121,9 @@ __device__ __forceinline__ double clip_p(double p, double smallp) {
 template <int NDIR, bool MHD>
 __device__ __forceinline__ double pthermal_raw(const double* u,
                                                const PhysConst& k) {
-  if (MHD) return pthermal_mhd_raw<NDIR>(u, k);
-  return pthermal_hd_raw<NDIR>(u, k);
+  const Rcp64 ir = rcp64(u[0]);
+  if (MHD) return pthermal_mhd_raw<NDIR>(u, ir, k);
+  return pthermal_hd_raw<NDIR>(u, ir, k);
 }
 
 // getcmax, src/vacphys0.t.mhd:79-116 (fast speed) / src/vacphys0.t.hd:72-100
@@ -88,21 +131,29 @@ template <int NDIR, bool MHD>
 __device__ __forceinline__ double cmax_fn(const double* u, int idim,
                                           const PhysConst& k, double smallp) {
   typedef Lay<NDIR, MHD> L;
+  const Rcp64 ir = rcp64(u[0]);
   if (MHD) {
-    double p = clip_p(pthermal_mhd_raw<NDIR>(u, k), smallp);
-    double cs2 = k.gamma * p / u[0];
+    double p = clip_p(pthermal_mhd_raw<NDIR>(u, ir, k), smallp);
+    double cs2 = div64(k.gamma * p, ir);
     double bb = u[L::B0 + 1] * u[L::B0 + 1];
 #pragma unroll
     for (int c = 2; c <= NDIR; c++) bb = bb + u[L::B0 + c] * u[L::B0 + c];
-    double cf2 = bb / u[0] + cs2;
+    double cf2 = div64(bb, ir) + cs2;
     double bi = u[L::B0 + 1 + idim];
-    return sqrt(0.5 * (cf2 + sqrt(cf2 * cf2 - 4.0 * cs2 * (bi * bi) / u[0]))) +
-           fabs(u[1 + idim] / u[0]);
+    // cf2*cf2 - 4*cs2*bi^2/rho
+    const double q = fma(-4.0, div64(cs2 * (bi * bi), ir), cf2 * cf2);
+    return sqrt(0.5 * (cf2 + sqrt(q))) + fabs(div64(u[1 + idim], ir));
   } else {
-    double p = clip_p(pthermal_hd_raw<NDIR>(u, k), smallp);
-    double cs = sqrt(k.gamma * p / u[0]);
-    return cs + fabs(u[1 + idim] / u[0]);
+    double p = clip_p(pthermal_hd_raw<NDIR>(u, ir, k), smallp);
+    double cs = sqrt(div64(k.gamma * p, ir));
+    return cs + fabs(div64(u[1 + idim], ir));
   }
+}
+
+// 0.0 + x: x, with -0 made +0 (an integer select instead of an addition)
+__device__ __forceinline__ double plus_zero(double x) {
+  const long long b = __double_as_longlong(x);
+  return b == (long long)0x8000000000000000ULL ? 0.0 : x;
 }
 
 // getflux + transport term, src/vacphys.mhd0.t:149-205 and
@@ -113,12 +164,12 @@ __device__ __forceinline__ void flux_fn(const double* u, int idim,
                                         const PhysConst& k, double smallp,
                                         double* f) {
   typedef Lay<NDIR, MHD> L;
-  const double rho = u[0];
-  const double v = u[1 + idim] / rho;
+  const Rcp64 ir = rcp64(u[0]);
+  const double v = div64(u[1 + idim], ir);
   if (MHD) {
-    const double pt = ptotal_mhd<NDIR>(u, k);
+    const double pt = ptotal_mhd<NDIR>(u, ir, k);
     const double bi = u[L::B0 + 1 + idim];
-    f[0] = 0.0 + v * u[0];
+    f[0] = plus_zero(v * u[0]);
 #pragma unroll
     for (int c = 1; c <= NDIR; c++) {
       double bk = u[L::B0 + c];
@@ -128,23 +179,22 @@ __device__ __forceinline__ void flux_fn(const double* u, int idim,
     double bm = u[L::B0 + 1] * u[1];
 #pragma unroll
     for (int c = 2; c <= NDIR; c++) bm = bm + u[L::B0 + c] * u[c];
-    f[L::E] = (u[1 + idim] * pt - bi * bm) / rho + v * u[L::E];
+    f[L::E] = div64(u[1 + idim] * pt - bi * bm, ir) + v * u[L::E];
 #pragma unroll
     for (int c = 1; c <= NDIR; c++) {
       if (c == idim + 1)
         f[L::B0 + c] = 0.0;
       else
-        f[L::B0 + c] = -u[c] / rho * bi + v * u[L::B0 + c];
+        f[L::B0 + c] = div64(-u[c], ir) * bi + v * u[L::B0 + c];
     }
   } else {
-    const double p = clip_p(pthermal_hd_raw<NDIR>(u, k), smallp);
-    f[0] = 0.0 + v * u[0];
+    const double p = clip_p(pthermal_hd_raw<NDIR>(u, ir, k), smallp);
+    f[0] = plus_zero(v * u[0]);
 #pragma unroll
     for (int c = 1; c <= NDIR; c++) {
-      double fk = (c == idim + 1) ? p : 0.0;
-      f[c] = fk + v * u[c];
+      f[c] = c == idim + 1 ? p + v * u[c] : plus_zero(v * u[c]);
     }
-    f[L::E] = u[1 + idim] / rho * p + v * u[L::E];
+    f[L::E] = v * p + v * u[L::E];  // m/rho*p is v*p
   }
 }
 
@@ -180,13 +230,51 @@ __device__ __forceinline__ double limiter_fn(int lim, double a, double b) {
   }
 }
 
+// Half the limited slope, 0.5 * limiter_fn, with the same bits.  The selects
+// and sign changes of minmod and woodward run on the integer ALUs: as
+// 64-bit integers, doubles of clear sign bit compare as their values do, and
+// where a and b differ in sign the result is zero.  What is left for the
+// FP64 pipe is woodward's (a+b)/4 or minmod's factor 1/2, of 8 to 10
+// operations (comparisons run there as well).  NaN and slopes that overflow
+// take limiter_fn itself.
+static __device__ __noinline__ double half_limiter_fn(int lim, double a, double b) {
+  return 0.5 * limiter_fn(lim, a, b);
+}
+__device__ __forceinline__ double hlimiter_fn(int lim, double a, double b) {
+  constexpr long long SIGN = (long long)0x8000000000000000ULL;
+  constexpr long long INF = 0x7ff0000000000000LL;
+  const long long ia = __double_as_longlong(a);
+  const long long sg = ia & SIGN;            // s = sign(1, a)
+  const long long xa = ia & ~SIGN;           // |a|
+  const long long xb = __double_as_longlong(b) ^ sg;  // s*b
+  if (lim == LIM_WOODWARD) {
+    const long long it = __double_as_longlong(0.25 * (b + a));
+    const long long xt = it ^ sg;            // s*0.25*(b+a)
+    long long r = xa < xb ? xa : xb;
+    r = r < xt ? r : xt;
+    // s*b = -0 is the smaller of the first pair, and of the second unless
+    // (a+b)/4 is a zero too
+    if (xb < 0) r = xb != SIGN ? 0 : xt > 0 ? SIGN : xt;
+    const bool plain = (it & ~SIGN) <= INF && r < 0x7fe0000000000000LL;  // 2*r stays finite
+    return plain ? __longlong_as_double(r ^ sg) : half_limiter_fn(lim, a, b);
+  }
+  if (lim == LIM_MINMOD) {
+    long long r = xa < xb ? xa : xb;
+    if (xb < 0) r = xb == SIGN ? SIGN : 0;
+    return (xb & ~SIGN) <= INF ? 0.5 * __longlong_as_double(r ^ sg)
+                               : half_limiter_fn(lim, a, b);
+  }
+  return half_limiter_fn(lim, a, b);
+}
+
 // The FP64 physics policy of the sweep templates (sweep_fp64.cu,
 // roe_fp64.cu): storage and arithmetic in IEEE double.
 struct PH64 {
   typedef double T;
   typedef double R;
-  static __device__ __forceinline__ R limiter(int lim, R a, R b) {
-    return limiter_fn(lim, a, b);
+  // 0.5 * limiter
+  static __device__ __forceinline__ R hlimiter(int lim, R a, R b) {
+    return hlimiter_fn(lim, a, b);
   }
   template <int NDIR, bool MHD>
   static __device__ __forceinline__ void flux(const R* u, int d,
@@ -211,7 +299,7 @@ struct PH64 {
   // qdt/dx(ix,idim) of addflux (src/vacgrid.t:676-677)
   static __device__ __forceinline__ R qdx(double qdt, const DevArrays& a,
                                           int d, int i) {
-    return qdt / a.dx[d][i];
+    return div_dx(qdt, a, d, i);
   }
   // cmaxC*two/(dx(ixC)+dx(jxC)) (src/vactvdlf.t:188-190)
   static __device__ __forceinline__ double cfl(R cm, const DevArrays& a,
@@ -228,6 +316,21 @@ struct PH64 {
     return qdt * g;
   }
   static __device__ __forceinline__ R qdiv(double q) { return q; }
+  // several quotients by one density, and quotients by dx(ix,idim)
+  typedef Rcp64 Den;
+  static __device__ __forceinline__ Den den(R b) { return rcp64(b); }
+  static __device__ __forceinline__ R div(R a, const Den& r) { return div64(a, r); }
+  static __device__ __forceinline__ R div_dx(R q, const DevArrays& a, int d, int i) {
+    const double dx = a.dx[d][i];
+    if (!a.rdx[d]) return q / dx;
+    const double2 r = reinterpret_cast<const double2*>(a.rdx[d])[i];
+    Rcp64 den;
+    den.b = dx;
+    den.y = r.x;
+    den.yl = r.y;
+    den.ok = exponent_within(dx, 100);
+    return div64(q, den);
+  }
 };
 
 }  // namespace vacgpu

@@ -135,6 +135,11 @@ struct PHMixed {
     }
   }
 
+  // 0.5 * limiter
+  static __device__ __forceinline__ float hlimiter(int lim, float a, float b) {
+    return 0.5f * limiter(lim, a, b);
+  }
+
   // getflux + transport (src/vacphys.mhd0.t:149-205, src/vacphys.t.hd:49-75)
   template <int NDIR, bool MHD>
   static __device__ __forceinline__ void flux(const float* u, int d,
@@ -304,6 +309,12 @@ struct PHMixed {
     return (float)(qdt * g);
   }
   static __device__ __forceinline__ float qdiv(double q) { return (float)q; }
+  typedef float Den;
+  static __device__ __forceinline__ Den den(float b) { return b; }
+  static __device__ __forceinline__ float div(float a, Den b) { return a / b; }
+  static __device__ __forceinline__ float div_dx(float q, const DevArrays& a, int d, int i) {
+    return q / a.dxf[d][i];
+  }
 };
 
 }  // namespace vacgpu

@@ -653,17 +653,17 @@ struct RoeSweep {
                                               const T* __restrict__ w1,
                                               const T* __restrict__ base,
                                               long long o, long long s, int d,
-                                              int ci, R smallp, double qsmallp,
+                                              const int* cl, R smallp, double qsmallp,
                                               D qdt, bool limit, R* F, Face& f,
                                               D* am) {
     R wL[NW], wR[NW];
-    S::face_states(a, w1, base, o, s, smallp, limit, wL, wR);
+    S::face_states(a, w1, base, o, s, d, cl, smallp, limit, wL, wR);
     R fL[NW], fR[NW];
     PH::template flux<NDIR, MHD>(wL, d, a.ph, smallp, fL);
     PH::template flux<NDIR, MHD>(wR, d, a.ph, smallp, fR);
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) F[iw] = R(0.5) * (fL[iw] + fR[iw]);
-    const R dxs = PH::dx(a.a, d, ci) + PH::dx(a.a, d, ci + 1);
+    const R dxs = PH::dx(a.a, d, cl[d]) + PH::dx(a.a, d, cl[d] + 1);
     decompose(a, wL, wR, d, qsmallp, qdt, dxs, f, am);
   }
 
@@ -702,7 +702,7 @@ struct RoeSweep {
       Face fs;
       R F[NW];
       D am[2];
-      face(a, w1, base, o, st[d], d, cl[d], R(ctrl->smallp), ctrl->smallp,
+      face(a, w1, base, o, st[d], d, cl, R(ctrl->smallp), ctrl->smallp,
            ctrl->dt, limit, F, fs, am);
       if (a.ph.courantpar > 0.0) {
         key[0] = dkey((double)am[0]);
@@ -953,8 +953,7 @@ struct RoeSweep {
       R wc[NW];
 #pragma unroll
       for (int iw = 0; iw < NW; iw++) wc[iw] = R(w1[off + iw * vs]);
-      S::add_sources(a, S::src_qdt(a, qdt), wc, w1 + off, st,
-                     c, acc);
+      S::add_sources(a, S::src_qdt(a, false), wc, w1 + off, st, c, acc);
     }
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) wout[off + iw * vs] = T(acc[iw]);

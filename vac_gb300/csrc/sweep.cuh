@@ -200,16 +200,16 @@ struct Sweep {
   }
 
   // qdt*(idimmax-idimmin+1)/ndim of the unsplit source call
-  // (src/vactvdlf.t:85,292):
-  // the reference's double expression on the FP64 path; formed in FP32 on
-  // the mixed one, whose sources take it rounded to FP32 anyway (GB300's
-  // FP64 pipe would spend a double division per cell on it)
-  static __device__ __forceinline__ double src_qdt(const SweepArgs& a,
-                                                   double qdt) {
+  // (src/vactvdlf.t:85,292; pred: qdt = dt/2, the predictor's): the
+  // reference's double expression on the FP64 path, formed with the step's
+  // dt (a division per cell here would go to the FP64 pipe); formed in FP32
+  // on the mixed one, whose sources take it rounded to FP32 anyway
+  static __device__ __forceinline__ double src_qdt(const SweepArgs& a, bool pred) {
+    const double dt = a.ctrl->dt;
     if constexpr (sizeof(R) == 4)
-      return (double)((float)qdt * (float)((a.d1 - a.d0) + 1) / (float)NDIM);
+      return (double)((float)(pred ? dt / 2 : dt) * (float)((a.d1 - a.d0) + 1) / (float)NDIM);
     else
-      return qdt * ((a.d1 - a.d0) + 1.0) / NDIM;
+      return a.ctrl->srcq[pred ? 0 : 1];
   }
 
   // addsource2 (src/vac.t:575-605): specialsource (uniform gravity,
@@ -238,19 +238,23 @@ struct Sweep {
 #pragma unroll
       for (int d = 0; d < NDIM; d++) {
         const T* q = wct + (long long)(L::B0 + 1 + d) * a.g.vs;
-        R gq = R(0.5) * (R(q[st[d]]) - R(q[-st[d]])) / PH::dx(a.a, d, c[d]);
-        divb = divb + gq;
+        const R df = R(q[st[d]]) - R(q[-st[d]]);
+        if constexpr (sizeof(R) == 8)  // divb + 0.5*df/dx
+          divb = fma(0.5, PH::div_dx(df, a.a, d, c[d]), divb);
+        else
+          divb = divb + R(0.5) * df / PH::dx(a.a, d, c[d]);
       }
       divb = PH::qdiv(qdt) * divb;
+      const typename PH::Den ir = PH::den(wc[0]);
       R mb = wc[1] * wc[L::B0 + 1];
 #pragma unroll
       for (int k = 2; k <= NDIR; k++) mb = mb + wc[k] * wc[L::B0 + k];
 #pragma unroll
       for (int k = 1; k <= NDIR; k++) {
         acc[k] = acc[k] - wc[L::B0 + k] * divb;
-        acc[L::B0 + k] = acc[L::B0 + k] - wc[k] / wc[0] * divb;
+        acc[L::B0 + k] = acc[L::B0 + k] - PH::div(wc[k], ir) * divb;
       }
-      acc[L::E] = acc[L::E] - mb / wc[0] * divb;
+      acc[L::E] = acc[L::E] - PH::div(mb, ir) * divb;
     }
   }
 
@@ -311,7 +315,7 @@ struct Sweep {
   // (a runtime one puts the face states in a stack frame)
   template <int d>
   static __device__ __forceinline__ void predict_dir(
-      const SweepArgs& a, const T* __restrict__ w, long long off,
+      const SweepArgs& a, const T* __restrict__ w, long long off, long long n,
       const long long* st, const int* c, double qdt, R smallp, const R* u,
       const R* pc, R* acc) {
     const long long vs = a.g.vs;
@@ -324,9 +328,9 @@ struct Sweep {
       to_prim(a, smallp, pp);
 #pragma unroll
       for (int iw = 0; iw < NW; iw++) {
-        R l = PH::limiter(a.ph.lim[iw], pp[iw] - pc[iw], pc[iw] - pm[iw]);
-        uR[iw] = pc[iw] - R(0.5) * l;
-        uL[iw] = pc[iw] + R(0.5) * l;
+        R l = PH::hlimiter(a.ph.lim[iw], pp[iw] - pc[iw], pc[iw] - pm[iw]);
+        uR[iw] = pc[iw] - l;
+        uL[iw] = pc[iw] + l;
       }
       to_cons(a, uR);
       to_cons(a, uL);
@@ -335,9 +339,10 @@ struct Sweep {
       for (int iw = 0; iw < NW; iw++) {
         R wm = R(w[off + iw * vs - st[d]]);
         R wp = R(w[off + iw * vs + st[d]]);
-        R l = PH::limiter(a.ph.lim[iw], wp - u[iw], u[iw] - wm);
-        uR[iw] = u[iw] - R(0.5) * l;
-        uL[iw] = u[iw] + R(0.5) * l;
+        R l = PH::hlimiter(a.ph.lim[iw], wp - u[iw], u[iw] - wm);
+        uR[iw] = u[iw] - l;
+        uL[iw] = u[iw] + l;
+        if (sizeof(R) == 8 && a.slopes) ((R*)a.slopes)[n + iw * a.g.ncell] = l;
       }
     }
     R fL[NW], fR[NW];
@@ -391,12 +396,12 @@ struct Sweep {
     }
     for (int d = a.d0; d <= a.d1; d++) {
       if (d == 0)
-        predict_dir<0>(a, w, off, st, c, qdt, smallp, u, pc, acc);
+        predict_dir<0>(a, w, off, n, st, c, qdt, smallp, u, pc, acc);
       else if (NDIM > 1 && d == 1)
-        predict_dir<(NDIM > 1 ? 1 : 0)>(a, w, off, st, c, qdt, smallp, u, pc,
+        predict_dir<(NDIM > 1 ? 1 : 0)>(a, w, off, n, st, c, qdt, smallp, u, pc,
                                         acc);
       else if (NDIM > 2)
-        predict_dir<(NDIM > 2 ? 2 : 0)>(a, w, off, st, c, qdt, smallp, u, pc,
+        predict_dir<(NDIM > 2 ? 2 : 0)>(a, w, off, n, st, c, qdt, smallp, u, pc,
                                         acc);
     }
     if (a.ph.sourceunsplit && !a.ph.src_hook) {
@@ -406,8 +411,7 @@ struct Sweep {
 #pragma unroll
         for (int iw = 0; iw < NW; iw++) u[iw] = pc[iw];
       }
-      add_sources(a, src_qdt(a, qdt), u, w + off, st, c,
-                  acc);
+      add_sources(a, src_qdt(a, true), u, w + off, st, c, acc);
     }
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) w1[off + iw * vs] = T(acc[iw]);
@@ -419,7 +423,7 @@ struct Sweep {
   // src/vactvdlf.t:325-362); the first order methods take wCT unlimited.
   static __device__ __forceinline__ void face_states(
       const SweepArgs& a, const T* __restrict__ w1, const T* __restrict__ base,
-      long long o, long long s, R smallp, bool limit, R* wL, R* wR) {
+      long long o, long long s, int d, const int* cl, R smallp, bool limit, R* wL, R* wR) {
     const long long vs = a.g.vs;
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) {
@@ -440,22 +444,32 @@ struct Sweep {
       to_prim(a, smallp, wR);
 #pragma unroll
       for (int iw = 0; iw < NW; iw++) {
-        R ldL = PH::limiter(a.ph.lim[iw], b1[iw] - b0[iw], b0[iw] - bm[iw]);
-        R ldR = PH::limiter(a.ph.lim[iw], b2[iw] - b1[iw], b1[iw] - b0[iw]);
-        wR[iw] = wR[iw] - R(0.5) * ldR;
-        wL[iw] = wL[iw] + R(0.5) * ldL;
+        R ldL = PH::hlimiter(a.ph.lim[iw], b1[iw] - b0[iw], b0[iw] - bm[iw]);
+        R ldR = PH::hlimiter(a.ph.lim[iw], b2[iw] - b1[iw], b1[iw] - b0[iw]);
+        wR[iw] = wR[iw] - ldR;
+        wL[iw] = wL[iw] + ldL;
       }
       to_cons(a, wL);
       to_cons(a, wR);
+    } else if (sizeof(R) == 8 && limit && a.slopes && cl[d] >= 2 && cl[d] <= a.g.nx[d]) {
+      // the predictor's slopes of the two mesh cells
+      const int m0 = cl[0] - a.g.gh[0], m1 = cl[1] - a.g.gh[1], m2 = cl[2] - a.g.gh[2];
+      const R* h = (const R*)a.slopes + ((long long)m2 * a.g.nx[1] + m1) * a.g.nx[0] + m0;
+      const long long ms = d == 0 ? 1 : d == 1 ? a.g.nx[0] : (long long)a.g.nx[0] * a.g.nx[1];
+#pragma unroll
+      for (int iw = 0; iw < NW; iw++) {
+        wR[iw] = wR[iw] - h[iw * a.g.ncell + ms];
+        wL[iw] = wL[iw] + h[iw * a.g.ncell];
+      }
     } else if (limit) {
 #pragma unroll
       for (int iw = 0; iw < NW; iw++) {
         const T* b = base + o + iw * vs;
         R bm = R(b[-s]), b0 = R(b[0]), b1 = R(b[s]), b2 = R(b[2 * s]);
-        R ldL = PH::limiter(a.ph.lim[iw], b1 - b0, b0 - bm);
-        R ldR = PH::limiter(a.ph.lim[iw], b2 - b1, b1 - b0);
-        wR[iw] = wR[iw] - R(0.5) * ldR;
-        wL[iw] = wL[iw] + R(0.5) * ldL;
+        R ldL = PH::hlimiter(a.ph.lim[iw], b1 - b0, b0 - bm);
+        R ldR = PH::hlimiter(a.ph.lim[iw], b2 - b1, b1 - b0);
+        wR[iw] = wR[iw] - ldR;
+        wL[iw] = wL[iw] + ldL;
       }
     }
   }
@@ -466,24 +480,31 @@ struct Sweep {
                                                 const T* __restrict__ w1,
                                                 const T* __restrict__ base,
                                                 long long o, long long s,
-                                                int d, R smallp, R* F) {
+                                                int d, const int* cl, R smallp, R* F) {
     R wL[NW], wR[NW];
-    face_states(a, w1, base, o, s, smallp, a.ph.typefull != VACGPU_TVDLF1, wL,
+    face_states(a, w1, base, o, s, d, cl, smallp, a.ph.typefull != VACGPU_TVDLF1, wL,
                 wR);
     R mean[NW];
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) mean[iw] = R(0.5) * (wL[iw] + wR[iw]);
     const R cmax = PH::template cmax<NDIR, MHD>(mean, d, a.ph, smallp);
 #pragma unroll
-    for (int iw = 0; iw < NW; iw++) wL[iw] = R(2) * mean[iw] - wR[iw];
+    for (int iw = 0; iw < NW; iw++) {
+      if constexpr (sizeof(R) == 8)
+        wL[iw] = fma(2.0, mean[iw], -wR[iw]);
+      else
+        wL[iw] = R(2) * mean[iw] - wR[iw];
+    }
     R fL[NW], fR[NW];
     PH::template flux<NDIR, MHD>(wL, d, a.ph, smallp, fL);
     PH::template flux<NDIR, MHD>(wR, d, a.ph, smallp, fR);
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) {
-      R f = R(0.5) * (fL[iw] + fR[iw]);
-      R diss = -cmax * R(0.5) * (wR[iw] - wL[iw]);
-      F[iw] = f + diss;
+      const R diss = -cmax * R(0.5) * (wR[iw] - wL[iw]);
+      if constexpr (sizeof(R) == 8)
+        F[iw] = fma(0.5, fL[iw] + fR[iw], diss);
+      else
+        F[iw] = R(0.5) * (fL[iw] + fR[iw]) + diss;
     }
     return cmax;
   }
@@ -513,7 +534,7 @@ struct Sweep {
       const long long st[3] = {1, g.P, g.plane};
       const long long o = gidx(g, cl[0], cl[1], cl[2]);
       R Ff[NW];
-      const R cm = face_flux(a, w1, base, o, st[d], d, R(ctrl->smallp), Ff);
+      const R cm = face_flux(a, w1, base, o, st[d], d, cl, R(ctrl->smallp), Ff);
       if (a.ph.courantpar > 0.0) key = dkey(PH::cfl(cm, a.a, d, cl[d]));
       const int nof = cl[d] == 1 ? a.ph.noflux[d][0]
                       : cl[d] == g.nx[d] + 1 ? a.ph.noflux[d][1] : 0;
@@ -567,8 +588,7 @@ struct Sweep {
       R wc[NW];
 #pragma unroll
       for (int iw = 0; iw < NW; iw++) wc[iw] = R(w1[off + iw * vs]);
-      add_sources(a, src_qdt(a, qdt), wc, w1 + off, st, c,
-                  acc);
+      add_sources(a, src_qdt(a, false), wc, w1 + off, st, c, acc);
     }
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) wout[off + iw * vs] = T(acc[iw]);
@@ -589,14 +609,13 @@ struct Sweep {
     const long long off = gidx(a.g, c[0], c[1], c[2]);
     const long long st[3] = {1, a.g.P, a.g.plane};
     const long long vs = a.g.vs;
-    const double qdt = pred ? ctrl->dt / 2 : ctrl->dt;
     R acc[NW], wc[NW];
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) {
       acc[iw] = R(w[off + iw * vs]);
       wc[iw] = R(wct[off + iw * vs]);
     }
-    add_sources(a, src_qdt(a, qdt), wc, wct + off, st, c, acc);
+    add_sources(a, src_qdt(a, pred != 0), wc, wct + off, st, c, acc);
 #pragma unroll
     for (int iw = 0; iw < NW; iw++) w[off + iw * vs] = T(acc[iw]);
   }

@@ -163,6 +163,7 @@ struct vacgpu_handle {
   int* poll;
   cudaEvent_t poll_ev[2];
   double* dx[3];
+  double* rdx[3];    // FP64 path: DevArrays::rdx
   float* dxf[3];
   std::vector<double> hdx[3];
   double volume;
@@ -366,11 +367,13 @@ void fill_ghosts(vacgpu_handle* h, const SweepArgs& a, void* w, int restore,
 
 SweepArgs make_args(vacgpu_handle* h, int d0, int d1) {
   SweepArgs a;
+  a.slopes = nullptr;
   a.g = h->g;
   a.ph = h->ph;
   for (int d = 0; d < 3; d++) {
     a.a.dx[d] = h->dx[d];
     a.a.dxf[d] = h->dxf[d];
+    a.a.rdx[d] = h->rdx[d];
   }
   a.ctrl = h->ctrl;
   a.etaf = h->etaf;
@@ -485,6 +488,11 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
   T* wout = (T*)h->buf[h->cur ^ 1];
   T* w1 = (T*)h->buf[2];
   const T* base = w;
+  // the half slopes go through the transfer buffer, which only transfers on
+  // this stream use otherwise
+  if (h->elem == 8 && h->p.dimsplit && h->p.typelimited == VACGPU_LIMITED_ORIGINAL &&
+      !h->ph.useprim)
+    a.slopes = h->stage;
   if (h->p.typelimited == VACGPU_LIMITED_PREDICTOR) base = w1;
   if (h->p.typelimited == VACGPU_LIMITED_PREVIOUS && h->p.dimsplit)
     base = (const T*)h->wold;
@@ -1131,7 +1139,11 @@ int vacgpu_create(const vacgpu_params* p, vacgpu_handle** out) {
   for (int d = 0; d < 3 && e == cudaSuccess; d++) {
     e = cudaMalloc(&h->xg[d], sizeof(double) * g.nG[d]);
     if (e == cudaSuccess) e = cudaMemset(h->xg[d], 0, sizeof(double) * g.nG[d]);
-    if (e == cudaSuccess) e = cudaMalloc(&h->dx[d], sizeof(double) * g.nG[d]);
+    // FP64: dx, padded to an even count, then the pairs of rdx
+    const int ne = (g.nG[d] + 1) & ~1;
+    if (e == cudaSuccess)
+      e = cudaMalloc(&h->dx[d], sizeof(double) * (h->elem == 8 ? 3 * ne : ne));
+    if (e == cudaSuccess && h->elem == 8) h->rdx[d] = h->dx[d] + ne;
     if (e == cudaSuccess) e = cudaMalloc(&h->dxf[d], sizeof(float) * g.nG[d]);
   }
   if (e == cudaSuccess && p->physics == VACGPU_PHYS_MHD && p->eqpar[1] < 0.0) {
@@ -1273,8 +1285,17 @@ int vacgpu_set_grid(vacgpu_handle* h, const double* x) {
       f[i] = (float)h->hdx[d][i];
       if (!(h->hdx[d][i] > 0.0)) return fail("grid spacing must be positive");
     }
-    CK(cudaMemcpy(h->dx[d], h->hdx[d].data(), sizeof(double) * (N + 4),
-                  cudaMemcpyHostToDevice));
+    std::vector<double> dr(h->hdx[d]);
+    if (h->rdx[d]) {
+      dr.resize((size_t)(h->rdx[d] - h->dx[d]) + 2 * (N + 4));
+      double* r = dr.data() + (h->rdx[d] - h->dx[d]);
+      for (int i = 0; i < N + 4; i++) {
+        const double b = h->hdx[d][i], y = 1.0 / b;
+        r[2 * i] = y;
+        r[2 * i + 1] = std::fma(-b, y, 1.0) * y;
+      }
+    }
+    CK(cudaMemcpy(h->dx[d], dr.data(), sizeof(double) * dr.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(h->dxf[d], f.data(), sizeof(float) * (N + 4),
                   cudaMemcpyHostToDevice));
     if (h->idxf[d]) {

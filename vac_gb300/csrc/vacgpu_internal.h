@@ -128,6 +128,7 @@ struct CtrlHead {
   double smallp;
   double dtgrav;
   double dtspecial;   // the user's getdt_special limit of this step (BIG: none)
+  double srcq[2];     // qdt*(idimmax-idimmin+1)/ndim of the predictor and corrector
   double src_qdt, src_qtc;  // qdt and qtC of the source call being issued
   double dtdiff;      // resistive diffusion dt limit (BIG without resistivity)
   double qt;          // time of the current ghost fill (specialbound hooks)
@@ -222,6 +223,9 @@ __host__ __device__ inline double dkey_inv(unsigned long long k) {
 struct DevArrays {
   const double* dx[3];  // dx over the ghost-extended range, per dimension
   const float* dxf[3];  // FP32 copies for the mixed path
+  // FP64 path: per dx the pair RN(1/dx), 1/dx - RN(1/dx) of Rcp64 (physics.cuh);
+  // nullptr: divisions by dx in full
+  const double* rdx[3];
 };
 
 // Launchers (sweep_fp64.cu, sweep_mixed.cu).  `w` is the state at the start
@@ -241,6 +245,10 @@ struct SweepArgs {
   // fluxes) variable-major
   void* faces;
   long long face_stride;
+  // FP64 split sweeps that limit the state itself: the predictor's half
+  // slopes of the mesh cells (mesh order, variable-major), which the face
+  // pass reads; nullptr: the face pass forms its slopes from the base
+  double* slopes;
   int ndir, mhd;
   int d0, d1;           // sweep dimensions (d0==d1 when split)
   int typelimited;
