@@ -8,6 +8,7 @@
 #include <mutex>
 #include <string>
 
+#include "ghost_images.cuh"
 #include "vacgpu_internal.h"
 
 using namespace vacgpu;
@@ -179,6 +180,7 @@ extern "C" int vacgpu_sweep_noalloc(const vacgpu_params* p, const double* w,
   s.typelimited = p->typelimited;
   s.faces = a.faces;
   s.face_stride = (long long)p->nw * face_count(g, idim);
+  s.images = ghost_images_apply(g, ph);
 
   cudaStream_t st = (cudaStream_t)stream;
   k_na_begin<<<1, NSLOT, 0, st>>>(a.ctrl, dt, p->smallp, p->ndim);
@@ -188,11 +190,11 @@ extern "C" int vacgpu_sweep_noalloc(const vacgpu_params* p, const double* w,
     launch_correct_fp64(s, w, w, w, wout, st);
   } else {
     launch_predict_fp64(s, w, a.w1, st);
-    launch_ghost_fp64(s, a.w1, st);
+    if (!s.images) launch_ghost_fp64(s, a.w1, st);
     const double* base = p->typelimited == VACGPU_LIMITED_PREDICTOR ? a.w1 : w;
     launch_correct_fp64(s, w, a.w1, base, wout, st);
   }
-  launch_ghost_fp64(s, wout, st);
+  if (!s.images) launch_ghost_fp64(s, wout, st);
   if (courantmax) k_na_end<<<1, NSLOT, 0, st>>>(a.ctrl, idim, courantmax);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)

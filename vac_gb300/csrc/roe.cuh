@@ -955,8 +955,7 @@ struct RoeSweep {
       for (int iw = 0; iw < NW; iw++) wc[iw] = R(w1[off + iw * vs]);
       S::add_sources(a, S::src_qdt(a, false), wc, w1 + off, st, c, acc);
     }
-#pragma unroll
-    for (int iw = 0; iw < NW; iw++) wout[off + iw * vs] = T(acc[iw]);
+    S::store_cell(a, wout, off, c, acc);
   }
 };
 
@@ -984,15 +983,17 @@ void launch_roe_instance(const SweepArgs& a, const typename PH::T* w,
   for (int d = a.d0; d <= a.d1; d++) {
     typename PH::R* buf =
         (typename PH::R*)a.faces + (long long)(d - a.d0) * a.face_stride;
-    const unsigned nbf = grid_for(face_count(a.g, d), 128);
+    const int ntf = split_threads(face_count(a.g, d));
+    const unsigned nbf = grid_for(face_count(a.g, d), ntf);
     if (d == 0)
-      k_roe_face<PH, NDIM, NDIR, MHD, 0><<<nbf, 128, 0, st>>>(a, w1, base, buf);
+      k_roe_face<PH, NDIM, NDIR, MHD, 0><<<nbf, ntf, 0, st>>>(a, w1, base, buf);
     else if (NDIM > 1 && d == 1)
-      k_roe_face<PH, NDIM, NDIR, MHD, (NDIM > 1 ? 1 : 0)><<<nbf, 128, 0, st>>>(a, w1, base, buf);
+      k_roe_face<PH, NDIM, NDIR, MHD, (NDIM > 1 ? 1 : 0)><<<nbf, ntf, 0, st>>>(a, w1, base, buf);
     else if (NDIM > 2)
-      k_roe_face<PH, NDIM, NDIR, MHD, (NDIM > 2 ? 2 : 0)><<<nbf, 128, 0, st>>>(a, w1, base, buf);
+      k_roe_face<PH, NDIM, NDIR, MHD, (NDIM > 2 ? 2 : 0)><<<nbf, ntf, 0, st>>>(a, w1, base, buf);
   }
-  k_correct_roe<PH, NDIM, NDIR, MHD><<<grid_for(a.g.ncell, 128), 128, 0, st>>>(a, w, w1, wout);
+  const int nt = split_threads(a.g.ncell);
+  k_correct_roe<PH, NDIM, NDIR, MHD><<<grid_for(a.g.ncell, nt), nt, 0, st>>>(a, w, w1, wout);
 }
 
 // (ndim, ndir, physics) instances; the MHD Roe solver needs ndir >= 2

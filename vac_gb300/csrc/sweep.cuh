@@ -6,6 +6,7 @@
 // Templated on a physics policy PH (storage type T, arithmetic type R and
 // the pointwise physics), the dimensionality and the physics module.
 #pragma once
+#include "ghost_images.cuh"
 #include "vacgpu_internal.h"
 
 namespace vacgpu {
@@ -19,7 +20,8 @@ __device__ __forceinline__ void atomic_min_key(unsigned long long* a,
   atomicMin(a, k);
 }
 
-// Block-wide max of an ordered key; thread 0 returns the result.
+// Block-wide max of an ordered key; thread 0 returns the result (blocks of
+// up to NT threads).
 template <int NT>
 __device__ __forceinline__ unsigned long long block_max_key(
     unsigned long long k, unsigned long long* sh) {
@@ -28,11 +30,12 @@ __device__ __forceinline__ unsigned long long block_max_key(
     unsigned long long v = __shfl_xor_sync(0xffffffffu, k, o);
     k = v > k ? v : k;
   }
+  if (blockDim.x <= 32) return k;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) sh[wid] = k;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int i = 1; i < NT / 32; i++) k = sh[i] > k ? sh[i] : k;
+    for (int i = 1; i < (int)blockDim.x / 32; i++) k = sh[i] > k ? sh[i] : k;
   }
   __syncthreads();
   return k;
@@ -291,6 +294,19 @@ struct Sweep {
     for (int iw = 0; iw < NW; iw++) u[iw] = R(w[o + iw * vs]);
   }
 
+  // the new value of the mesh cell c, with its ghost images where the launch
+  // fills the ghost cells (SweepArgs::images)
+  static __device__ __forceinline__ void store_cell(const SweepArgs& a, T* __restrict__ w,
+                                                    long long off, const int* c, const R* acc) {
+#pragma unroll
+    for (int iw = 0; iw < NW; iw++) w[off + iw * a.g.vs] = T(acc[iw]);
+    if (!a.images) return;
+    bool near = false;
+#pragma unroll
+    for (int d = 0; d < NDIM; d++) near = near || c[d] < 4 || c[d] >= a.g.nx[d];
+    if (near) write_ghost_images<NDIM, NW>(a.g, a.ph, w, c, off, acc);
+  }
+
   // useprimitive's in-place round trip of the limiter base over the ghost
   // box: out = conserve(primitive(w)) (src/vactvdlf.t:325-330,357-362).
   static __device__ void roundtrip(const SweepArgs& a, const T* __restrict__ w,
@@ -413,8 +429,7 @@ struct Sweep {
       }
       add_sources(a, src_qdt(a, true), u, w + off, st, c, acc);
     }
-#pragma unroll
-    for (int iw = 0; iw < NW; iw++) w1[off + iw * vs] = T(acc[iw]);
+    store_cell(a, w1, off, c, acc);
   }
 
   // Face states of upwindLR (src/vactvdlf.t:302-367) at the face between
@@ -590,8 +605,7 @@ struct Sweep {
       for (int iw = 0; iw < NW; iw++) wc[iw] = R(w1[off + iw * vs]);
       add_sources(a, src_qdt(a, false), wc, w1 + off, st, c, acc);
     }
-#pragma unroll
-    for (int iw = 0; iw < NW; iw++) wout[off + iw * vs] = T(acc[iw]);
+    store_cell(a, wout, off, c, acc);
   }
 
   // addsource (src/vac.t:575-605 after specialsource) as a pass of its own
@@ -1038,13 +1052,13 @@ __global__ void __launch_bounds__(128)
 template <class PH, int NDIM, int NDIR, bool MHD>
 void launch_face_dir(const SweepArgs& a, const typename PH::T* w1,
                      const typename PH::T* base, int d, typename PH::R* F,
-                     unsigned nb, cudaStream_t st) {
+                     unsigned nb, int nt, cudaStream_t st) {
   if (d == 0)
-    k_face<PH, NDIM, NDIR, MHD, 0><<<nb, 128, 0, st>>>(a, w1, base, F);
+    k_face<PH, NDIM, NDIR, MHD, 0><<<nb, nt, 0, st>>>(a, w1, base, F);
   else if (NDIM > 1 && d == 1)
-    k_face<PH, NDIM, NDIR, MHD, (NDIM > 1 ? 1 : 0)><<<nb, 128, 0, st>>>(a, w1, base, F);
+    k_face<PH, NDIM, NDIR, MHD, (NDIM > 1 ? 1 : 0)><<<nb, nt, 0, st>>>(a, w1, base, F);
   else if (NDIM > 2)
-    k_face<PH, NDIM, NDIR, MHD, (NDIM > 2 ? 2 : 0)><<<nb, 128, 0, st>>>(a, w1, base, F);
+    k_face<PH, NDIM, NDIR, MHD, (NDIM > 2 ? 2 : 0)><<<nb, nt, 0, st>>>(a, w1, base, F);
 }
 
 template <class PH, int NDIM, int NDIR, bool MHD>
@@ -1122,12 +1136,21 @@ inline unsigned grid_for(long long n, int nt) {
   return (unsigned)((n + nt - 1) / nt);
 }
 
+// Threads per block of the predictor, face and cell passes: one warp where
+// blocks of four would be fewer than eight per SM (152), so the last blocks
+// leave no SM idle while others run two -- and a grid of few cells is spread
+// over more SMs (the FP64 pipe of one SM takes 6 us for the faces of 128
+// cells).  With that and the ghost images in the passes a 200^2 MHD step in
+// FP64 takes 125 us (158 before), one of 100 cells in 1-D 25 us (29).
+inline int split_threads(long long n) { return n < 8LL * 152 * 128 ? 32 : 128; }
+
 template <class PH>
 struct Launch {
   typedef typename PH::T T;
   static void predict(const SweepArgs& a, const T* w, T* w1, cudaStream_t st) {
-    unsigned nb = grid_for(a.g.ncell, 128);
-#define KC(D, C, M) k_predict<PH, D, C, M><<<nb, 128, 0, st>>>(a, w, w1)
+    const int nt = split_threads(a.g.ncell);
+    unsigned nb = grid_for(a.g.ncell, nt);
+#define KC(D, C, M) k_predict<PH, D, C, M><<<nb, nt, 0, st>>>(a, w, w1)
     VACGPU_DISPATCH(a, KC);
 #undef KC
   }
@@ -1136,13 +1159,15 @@ struct Launch {
                       const T* base, T* wout, cudaStream_t st) {
     for (int d = a.d0; d <= a.d1; d++) {
       typename PH::R* F = (typename PH::R*)a.faces + (long long)(d - a.d0) * a.face_stride;
-      const unsigned nbf = grid_for(face_count(a.g, d), 128);
-#define KC(D, C, M) launch_face_dir<PH, D, C, M>(a, w1, base, d, F, nbf, st)
+      const int ntf = split_threads(face_count(a.g, d));
+      const unsigned nbf = grid_for(face_count(a.g, d), ntf);
+#define KC(D, C, M) launch_face_dir<PH, D, C, M>(a, w1, base, d, F, nbf, ntf, st)
       VACGPU_DISPATCH(a, KC);
 #undef KC
     }
-    const unsigned nb = grid_for(a.g.ncell, 128);
-#define KC(D, C, M) k_correct<PH, D, C, M><<<nb, 128, 0, st>>>(a, w, w1, wout)
+    const int nt = split_threads(a.g.ncell);
+    const unsigned nb = grid_for(a.g.ncell, nt);
+#define KC(D, C, M) k_correct<PH, D, C, M><<<nb, nt, 0, st>>>(a, w, w1, wout)
     VACGPU_DISPATCH(a, KC);
 #undef KC
   }

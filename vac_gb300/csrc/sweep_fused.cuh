@@ -34,6 +34,7 @@
 #pragma once
 #include <cuda.h>
 
+#include "ghost_images.cuh"
 #include "physics_mixed.cuh"
 #include "vacgpu_internal.h"
 
@@ -543,52 +544,9 @@ struct Fused {
     return b;
   }
 
-  // Ghost-cell preimages of the mesh index gi along one dimension (n cells,
-  // ghost-range indices 0..n+3, n >= 4): up to two ghost positions p1, p2
-  // whose boundary map lands on gi, and the 'asymm' sign mask of each.
-  // periodic: gi-n for gi >= n, gi+n for gi < 4; cont: 0 and 1 for gi = 2,
-  // n+2 and n+3 for gi = n+1; symm/asymm: 3-gi for gi < 4, 2n+3-gi for
-  // gi >= n (negated for 'asymm' variables).
-  static __device__ __forceinline__ int preimages(const FusedArgs& a, int d,
-                                                  int gi, int& p1, int& f1,
-                                                  int& p2) {
-    const int n = a.g.nx[d];
-    const int mlo = a.ph.gmap[d][0], mhi = a.ph.gmap[d][1];
-    p1 = p2 = gi;
-    f1 = 0;
-    if (gi < 4) {
-      if (mlo == GMAP_CONT && gi == 2) {
-        p1 = 0;
-        p2 = 1;
-        return 2;
-      }
-      if (mlo == GMAP_MIRROR) {
-        p1 = 3 - gi;
-        f1 = a.ph.asym[d][0];
-        return 1;
-      }
-      if (mhi == GMAP_PERIODIC) {
-        p1 = gi + n;
-        return 1;
-      }
-    }
-    if (gi >= n) {
-      if (mhi == GMAP_CONT && gi == n + 1) {
-        p1 = n + 2;
-        p2 = n + 3;
-        return 2;
-      }
-      if (mhi == GMAP_MIRROR) {
-        p1 = 2 * n + 3 - gi;
-        f1 = a.ph.asym[d][1];
-        return 1;
-      }
-      if (mlo == GMAP_PERIODIC) {
-        p1 = gi - n;
-        return 1;
-      }
-    }
-    return 0;
+  static __device__ __forceinline__ int preimages(const FusedArgs& a, int d, int gi, int& p1,
+                                                  int& f1, int& p2) {
+    return ghost_preimages(a.g, a.ph, d, gi, p1, f1, p2);
   }
 
   // getboundary of the new state, done by its sources: every ghost cell

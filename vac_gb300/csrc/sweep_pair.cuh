@@ -228,42 +228,6 @@ __device__ __forceinline__ f2 p_hlim(f2 a, f2 b, const PairK& k) {
 
 // ------------------------------------------------------------ the kernel
 
-// getboundary's ghost images of one new cell value per variable (scalar,
-// one lane): the composition of the region copies of src/vacgrid.t:195-413
-// as in Fused::ghost_images (NDIM = 2: gc[2] = 0 and no z images).
-template <int NW, int NDIM = 3>
-__device__ __forceinline__ void pair_ghost_images(const FusedArgs& a,
-                                                  const int* gc, long long off,
-                                                  const float* acc) {
-  const DevGrid& g = a.g;
-  int x1, x2, fx, y1 = 0, y2 = 0, fy = 0, z1 = 0, z2 = 0, fz = 0;
-  typedef Fused<3, 0, true, PREC_FF, LIMC_MINMOD> FX;
-  const int nx_ = 1 + FX::preimages(a, 0, gc[0], x1, fx, x2);
-  const int ny_ = 1 + FX::preimages(a, 1, gc[1], y1, fy, y2);
-  const int nz_ = NDIM == 3 ? 1 + FX::preimages(a, 2, gc[2], z1, fz, z2) : 1;
-#pragma unroll 1
-  for (int k = 0; k < nz_; k++) {
-    const int pz = k == 0 ? gc[2] : (k == 1 ? z1 : z2);
-    const int sz = k == 1 ? fz : 0;
-#pragma unroll 1
-    for (int jj = 0; jj < ny_; jj++) {
-      const int py = jj == 0 ? gc[1] : (jj == 1 ? y1 : y2);
-      const int sy = jj == 1 ? fy : 0;
-      const long long orow =
-          off + (long long)(pz - gc[2]) * g.plane + (long long)(py - gc[1]) * g.P;
-#pragma unroll 1
-      for (int i = 0; i < nx_; i++) {
-        if ((i | jj | k) == 0) continue;
-        const int px = i == 0 ? gc[0] : (i == 1 ? x1 : x2);
-        const int fl = (i == 1 ? fx : 0) ^ sy ^ sz;
-        const long long o = orow + (px - gc[0]);
-#pragma unroll
-        for (int v = 0; v < NW; v++) a.wout[o + v * g.vs] = ((fl >> v) & 1) ? -acc[v] : acc[v];
-      }
-    }
-  }
-}
-
 // One split sweep along D of a 3-D grid, two cells per thread.  GEN:
 // the general form (gravity, non-periodic faces, sources or the CFL
 // maximum switched off); false: the common case -- every face periodic,
@@ -399,7 +363,7 @@ struct PairSweep {
       float s[NW];
 #pragma unroll
       for (int v = 0; v < NW; v++) s[v] = h ? f2hi(acc[v]) : f2lo(acc[v]);
-      pair_ghost_images<NW>(a, c2, off + h, s);
+      write_ghost_images<3, NW>(a.g, a.ph, a.wout, c2, off + h, s);
     }
   }
 

@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "ghost_images.cuh"
 #include "vacgpu_internal.h"
 
 using namespace vacgpu;
@@ -368,6 +369,7 @@ void fill_ghosts(vacgpu_handle* h, const SweepArgs& a, void* w, int restore,
 SweepArgs make_args(vacgpu_handle* h, int d0, int d1) {
   SweepArgs a;
   a.slopes = nullptr;
+  a.images = 0;
   a.g = h->g;
   a.ph = h->ph;
   for (int d = 0; d < 3; d++) {
@@ -481,6 +483,25 @@ void source_hook(vacgpu_handle* h, const SweepArgs& a, int pred, int half, const
   kend(h);
 }
 
+// getboundary of a pass's output where the pass has not filled its ghost
+// cells itself, keeppositive first when smallfix; qtmode: the fill's qt
+void after_pass(vacgpu_handle* h, const SweepArgs& a, void* w, int qtmode) {
+  if (a.images) return;
+  kbegin(h, VACGPU_K_GHOST);
+  if (h->p.smallfix) {
+    if (h->elem == 8)
+      launch_keeppositive_fp64(a, (double*)w, h->st);
+    else if (h->pmode == 1)
+      launch_keeppositive_mixedf64(a, (float*)w, h->st);
+    else if (h->pmode == 2)
+      launch_keeppositive_mixedf32(a, (float*)w, h->st);
+    else
+      launch_keeppositive_mixed(a, (float*)w, h->st);
+  }
+  fill_ghosts(h, a, w, 1, qtmode);
+  kend(h);
+}
+
 template <typename T>
 void run_sweep(vacgpu_handle* h, int d0, int d1) {
   SweepArgs a = make_args(h, d0, d1);
@@ -493,6 +514,9 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
   if (h->elem == 8 && h->p.dimsplit && h->p.typelimited == VACGPU_LIMITED_ORIGINAL &&
       !h->ph.useprim)
     a.slopes = h->stage;
+  // the passes fill the ghost cells of their output, unless something else
+  // changes it first (keeppositive, the user's source)
+  a.images = !h->p.smallfix && !h->src_fn && ghost_images_apply(h->g, h->ph);
   if (h->p.typelimited == VACGPU_LIMITED_PREDICTOR) base = w1;
   if (h->p.typelimited == VACGPU_LIMITED_PREVIOUS && h->p.dimsplit)
     base = (const T*)h->wold;
@@ -533,27 +557,14 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
                            (const float*)w, (float*)wout, h->st);
     kend(h);
     source_hook<T>(h, a, 0, 0, w, wout);
-    if (h->p.smallfix) {
-      kbegin(h, VACGPU_K_GHOST);
-      if (sizeof(T) == 8)
-        launch_keeppositive_fp64(a, (double*)wout, h->st);
-      else
-        launch_keeppositive_mixed(a, (float*)wout, h->st);
-      kend(h);
-    }
-    kbegin(h, VACGPU_K_GHOST);
-    fill_ghosts(h, a, wout, 1, 2);
-    kend(h);
+    after_pass(h, a, wout, 2);
   } else if (sizeof(T) == 8) {
     if (h->p.sourceunsplit) eta_hook(h, a, w, 0);
     kbegin(h, VACGPU_K_PREDICT);
     launch_predict_fp64(a, (const double*)w, (double*)w1, h->st);
     kend(h);
     source_hook<T>(h, a, 1, 0, w, w1);
-    kbegin(h, VACGPU_K_GHOST);
-    if (h->p.smallfix) launch_keeppositive_fp64(a, (double*)w1, h->st);
-    fill_ghosts(h, a, w1, 1, 1);
-    kend(h);
+    after_pass(h, a, w1, 1);
     if (h->p.sourceunsplit) eta_hook(h, a, w1, 0);
     kbegin(h, VACGPU_K_CORRECT);
     if (roe)
@@ -564,10 +575,7 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
                           (const double*)base, (double*)wout, h->st);
     kend(h);
     source_hook<T>(h, a, 0, 1, (const T*)w1, wout);
-    kbegin(h, VACGPU_K_GHOST);
-    if (h->p.smallfix) launch_keeppositive_fp64(a, (double*)wout, h->st);
-    fill_ghosts(h, a, wout, 1, 2);
-    kend(h);
+    after_pass(h, a, wout, 2);
   } else if (h->fused && h->pmode == 0 && d0 == d1 && !h->src_fn) {
     kbegin(h, VACGPU_K_SWEEP);
     // the fused sweep also writes the ghost cells of its output
@@ -586,10 +594,7 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
   launch_predict_##SUF(a, fw, fw1, h->st);              \
   kend(h);                                              \
   source_hook<T>(h, a, 1, 0, w, w1);                    \
-  kbegin(h, VACGPU_K_GHOST);                            \
-  if (h->p.smallfix) launch_keeppositive_##SUF(a, fw1, h->st); \
-  fill_ghosts(h, a, fw1, 1, 1);                         \
-  kend(h);                                              \
+  after_pass(h, a, fw1, 1);                             \
   if (h->p.sourceunsplit) eta_hook(h, a, fw1, 0);       \
   kbegin(h, VACGPU_K_CORRECT);                          \
   if (roe)                                              \
@@ -598,10 +603,7 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
     launch_correct_##SUF(a, fwc, fw1, fb, fo, h->st);   \
   kend(h);                                              \
   source_hook<T>(h, a, 0, 1, (const T*)w1, wout);       \
-  kbegin(h, VACGPU_K_GHOST);                            \
-  if (h->p.smallfix) launch_keeppositive_##SUF(a, fo, h->st); \
-  fill_ghosts(h, a, fo, 1, 2);                          \
-  kend(h);
+  after_pass(h, a, fo, 2);
     switch (h->pmode) {
       case 1: MIXED_SWEEP(mixedf64) break;
       case 2: MIXED_SWEEP(mixedf32) break;

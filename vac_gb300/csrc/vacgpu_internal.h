@@ -249,6 +249,9 @@ struct SweepArgs {
   // slopes of the mesh cells (mesh order, variable-major), which the face
   // pass reads; nullptr: the face pass forms its slopes from the base
   double* slopes;
+  // the predictor and cell passes write the ghost images of their output
+  // (ghost_images.cuh); otherwise the caller fills its ghost cells
+  int images;
   int ndir, mhd;
   int d0, d1;           // sweep dimensions (d0==d1 when split)
   int typelimited;
