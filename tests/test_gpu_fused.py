@@ -244,3 +244,28 @@ def test_z_chunk_by_size_is_invisible(gpu_lib, monkeypatch, nx, lim, bc):
         e.close()
     assert out[0][0] == out[1][0]
     assert np.array_equal(out[0][1].view(np.uint64), out[1][1].view(np.uint64))
+
+
+
+@pytest.mark.parametrize("nx,bc", [((33, 18, 9), "cont"), ((45, 9, 17), "symm"),
+                                   ((31, 12, 10), "cont"), ((32, 12, 10), "cont")])
+def test_fused_odd_columns(gpu_lib, monkeypatch, nx, bc):
+    """MHD on a box cut out of the random modes, whose outflow or reflecting
+    x faces carry B_x: with an odd mesh width the last column shares its pair
+    with a ghost column."""
+    s = inistate.random_modes(max(nx), seed=8, p0=0.5)
+    s.x = inistate.domain_grid(nx, (0.0,) * 3, tuple(n / max(nx) for n in nx))
+    s.w = np.ascontiguousarray(s.w[:, :nx[0], :nx[1], :nx[2]])
+    s.nx = nx
+    p = inistate.params_for(s, limiter="minmod", bc=bc, precision=abi.PREC_MIXED)
+    if bc == "symm":
+        reflecting(p, 3)
+    out = []
+    for fused in ("1", "0"):
+        monkeypatch.setenv("VACGPU_FUSED", fused)
+        e = Engine(p, s.x, s.w)
+        e.step(1)
+        assert (e.kernel_stats()["sweep"][0] > 0) == (fused == "1")
+        out.append(e.state())
+        e.close()
+    assert max(rel_l1(out[0], out[1])) <= FUSED_VS_SPLIT, rel_l1(out[0], out[1])

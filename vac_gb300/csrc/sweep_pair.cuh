@@ -569,6 +569,13 @@ struct PairSweep {
                         gfix(oh, sh2, v, a.periodic_mask[AM], a.asymm_hi[AM]));
           }
         }
+        // an odd mesh width: the first ghost column is the second cell of the
+        // last pair, whose B_x the first cell's div B takes from registers
+        if (fix_x && ix0 + 1 == nX) {
+          float lo, hi;
+          f2u(w1[5], lo, hi);
+          w1[5] = f2m(lo, gfix(hi, lo, 5, a.periodic_mask[0], a.asymm_hi[0]));
+        }
         bz = w1[5 + AM];
         if (ring) {
           st2(wb(sm, j, 0, ly, lx0), w1[5]);
