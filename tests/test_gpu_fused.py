@@ -269,3 +269,57 @@ def test_fused_odd_columns(gpu_lib, monkeypatch, nx, bc):
         out.append(e.state())
         e.close()
     assert max(rel_l1(out[0], out[1])) <= FUSED_VS_SPLIT, rel_l1(out[0], out[1])
+
+
+ROE_CASES = [
+    ("rm3-periodic", (40, 33, 36), "woodward", "periodic", {}),
+    ("rm3-cont", (33, 18, 9), "minmod", "cont", {}),
+    ("rm3-reflect", (30, 20, 17), "woodward", "symm", {}),
+    ("rm3-nodivbwave", (31, 16, 24), "minmod", "periodic", {"divbwave": 0}),
+    ("rm3-nopowell", (32, 24, 16), "woodward", "periodic", {"divbfix": 0}),
+    ("rm2-periodic", (61, 50), "woodward", "periodic", {}),
+    ("rm2-cont", (130, 23), "minmod", "cont", {}),
+    ("rm2-reflect", (60, 64), "woodward", "symm", {"divbwave": 0}),
+]
+
+
+@pytest.mark.parametrize("name,nx,lim,bc,opt", ROE_CASES, ids=[c[0] for c in ROE_CASES])
+def test_fused_roe_against_oracle_and_split(gpu_lib, monkeypatch, name, nx, lim, bc, opt):
+    """'tvdmu' on the fused sweeps (ideal MHD, no entropy fix): within the
+    mixed tolerance of the FP64 oracle, and within FP32 rounding (twice the
+    TVDLF bound: eight waves' products in another order) of the split Roe
+    kernels; an entropy fix keeps the split kernels."""
+    nd = len(nx)
+    s = inistate.random_modes(max(nx), seed=8, p0=0.5, ndim=nd)
+    s.x = inistate.domain_grid(nx, (0.0,) * nd, tuple(n / max(nx) for n in nx))
+    s.w = np.ascontiguousarray(s.w[(slice(None),) + tuple(slice(0, n) for n in nx)])
+    s.nx = nx
+    p64 = inistate.params_for(s, limiter=lim, bc=bc)
+    pm = inistate.params_for(s, limiter=lim, bc=bc, precision=abi.PREC_MIXED)
+    for p in (p64, pm):
+        p.typefull = abi.TVDMU
+        for k, v in opt.items():
+            setattr(p, k, v)
+        if bc == "symm":
+            reflecting(p, nd)
+    # two steps against the walls: the oracle's pressure is negative after four
+    n = 2 if bc == "symm" else 8
+    o = Oracle(p64, s.x, s.w)
+    o.step(n)
+    out = []
+    for fused in ("1", "0"):
+        monkeypatch.setenv("VACGPU_FUSED", fused)
+        e = Engine(pm, s.x, s.w)
+        e.step(n)
+        assert (e.kernel_stats()["sweep"][0] > 0) == (fused == "1")
+        assert abs(e.t - o.t) <= 1e-6 * o.t
+        out.append(e.state())
+        assert max(rel_l1(out[-1], o.state())) <= MIXED_REL_L1
+        assert e.nerror() == o.nerror()
+        e.close()
+    assert max(rel_l1(out[0], out[1])) <= 2 * FUSED_VS_SPLIT
+    monkeypatch.setenv("VACGPU_FUSED", "1")
+    pm.typeentropy[0] = abi.ENTROPY_HARTEN
+    e = Engine(pm, s.x, s.w)
+    e.step(2)
+    assert e.kernel_stats()["sweep"][0] == 0

@@ -61,6 +61,24 @@ static void launch_one(const CUtensorMap* map, const FusedArgs& a, dim3 grid,
     launch_lim<NDIM, D, MHD, LIMC_RUNTIME>(map, a, grid, st);
 }
 
+bool pair_applies(const FusedArgs& a, bool mhd);
+bool line2_applies(const FusedArgs& a, bool mhd);
+
+// The fused sweeps with the Roe dissipation of 'tvdmu': ideal MHD without an
+// entropy fix (the fixes modify the normalised eigenvalues, which the split
+// kernels keep), on the grids of the two-cells-per-thread kernels alone.
+// (HD stays on the split kernels, whose average is in double.)
+bool fused_roe_applies(const DevGrid& g, const DevPhys& ph, int ndir, bool mhd) {
+  if (ph.typefull != VACGPU_TVDMU || !mhd || ndir != g.ndim) return false;
+  for (int il = 0; il < 2 + 2 * ndir; il++)
+    if (ph.typeentropy[il] != VACGPU_ENTROPY_NUL) return false;
+  FusedArgs a;
+  memset(&a, 0, sizeof(a));
+  a.g = g;
+  a.ph = ph;
+  return g.ndim == 3 ? pair_applies(a, mhd) : g.ndim == 2 && line2_applies(a, mhd);
+}
+
 bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win, float* wout,
                         const float* const* idxf, int nzc, cudaStream_t st) {
   const int nd = s.g.ndim;

@@ -15,7 +15,7 @@ bool pair_general(const FusedArgs& a, bool mhd);
 
 // One work item per warp: item = strip + nstrips * chunk of `rows` rows.
 // register bound: four CTAs per SM for HD (128 registers), two for MHD
-template <int D, bool MHD, int LIMC, bool GEN>
+template <int D, bool MHD, int LIMC, bool GEN, bool ROE>
 __global__ void __launch_bounds__(L2_NT, MHD ? 2 : 4)
     k_sweep_line2(const FusedArgs a, const float* __restrict__ win, int nstrips, int nitems,
                   int rows) {
@@ -25,8 +25,8 @@ __global__ void __launch_bounds__(L2_NT, MHD ? 2 : 4)
   __shared__ __align__(16) float ring[L2_NT / 32][RF];
   const int sx = item % nstrips, ch = item / nstrips;
   const int gya = 2 + ch * rows, gyb = min(gya + rows, a.g.nx[1] + 2);
-  Line2<D, MHD, LIMC, GEN>::run(a, win, a.wout, ring[threadIdx.x >> 5], sx, gya, gyb,
-                                (unsigned)item);
+  Line2<D, MHD, LIMC, GEN, ROE>::run(a, win, a.wout, ring[threadIdx.x >> 5], sx, gya, gyb,
+                                     (unsigned)item);
 }
 
 // Batched grids: each warp takes items gw, gw + W, ... of the work list
@@ -93,13 +93,13 @@ static int line2_items(int D, bool mhd, const DevGrid& g, int rows, int* nstrips
   return *nstrips * ((g.nx[1] + rows - 1) / rows);
 }
 
-template <int D, bool MHD, int LIMC, bool GEN>
+template <int D, bool MHD, int LIMC, bool GEN, bool ROE = false>
 static void launch_l2(const FusedArgs& a, const float* win, cudaStream_t st) {
   int ns;
   const int rows = line2_rows(D, MHD, a.g);
   const int n = line2_items(D, MHD, a.g, rows, &ns);
   const int per = L2_NT / 32;
-  k_sweep_line2<D, MHD, LIMC, GEN><<<(n + per - 1) / per, L2_NT, 0, st>>>(a, win, ns, n, rows);
+  k_sweep_line2<D, MHD, LIMC, GEN, ROE><<<(n + per - 1) / per, L2_NT, 0, st>>>(a, win, ns, n, rows);
 }
 
 bool launch_sweep_line2(const FusedArgs& a, const float* win, int D, bool mhd,
@@ -107,6 +107,19 @@ bool launch_sweep_line2(const FusedArgs& a, const float* win, int D, bool mhd,
   if (!line2_applies(a, mhd)) return false;
   const bool gen = pair_general(a, mhd);
   const int l0 = a.ph.lim[0];
+  if (a.ph.typefull == VACGPU_TVDMU) {
+#define L2R(DD, L)                                                           \
+  if (D == DD && l0 == VACGPU_LIM_##L) {                                     \
+    if (gen)                                                                 \
+      launch_l2<DD, true, LIMC_##L, true, true>(a, win, st);                 \
+    else                                                                     \
+      launch_l2<DD, true, LIMC_##L, false, true>(a, win, st);                \
+    return true;                                                             \
+  }
+    L2R(0, WOODWARD) L2R(0, MINMOD) L2R(1, WOODWARD) L2R(1, MINMOD)
+#undef L2R
+    return false;
+  }
 #define L2G(DD, M, L)                                                        \
   {                                                                          \
     if (gen)                                                                 \

@@ -53,7 +53,8 @@ constexpr int L2_ROWF = 68;
 // floats of one warp's row-staging ring for nw variables
 __host__ __device__ constexpr int line2_ring_floats(int nw) { return L2_RING * nw * L2_ROWF; }
 
-template <int D, bool MHD, int LIMC, bool GEN>
+// (ROE: as PairSweep's)
+template <int D, bool MHD, int LIMC, bool GEN, bool ROE = false>
 struct Line2 {
   static constexpr int NW = MHD ? 6 : 4;
   static constexpr int E = 3;                  // e
@@ -204,10 +205,19 @@ struct Line2 {
   }
 
   // TVDLF face flux 2F = F(L) + F(R) - cmax (R - L) of a pair of faces
-  static __device__ __forceinline__ f2 face(const f2* L, const f2* R, const PairK& k, f2* G) {
+  static __device__ __forceinline__ f2 face(const FusedArgs& a, const f2* L, const f2* R,
+                                            const PairK& k, f2* G, f2& cm2) {
     f2 fL[NW], fR[NW], pL, pR, riL, riR;
     p_flux<D, MHD, 2>(L, k, fL, pL, riL);
     p_flux<D, MHD, 2>(R, k, fR, pR, riR);
+    if constexpr (ROE) {
+#pragma unroll
+      for (int v = 0; v < NW; v++) G[v] = fL[v] + fR[v];
+      f2 cm1;
+      p_roe_dissipation<D, 2>(L, R, pL, pR, riL, riR, k, f2s(a.ph.c2gf), a.ph.divbwave, G, cm1,
+                              cm2);
+      return cm1;
+    }
     f2 M[NW];
     M[0] = k.half * (L[0] + R[0]);
     M[1 + D] = k.half * (L[1 + D] + R[1 + D]);
@@ -300,6 +310,20 @@ struct Line2 {
     qmax = f2m(ql, qh);
   }
 
+  // the warp's maximum of qmax into the slots of `to`
+  static __device__ __forceinline__ void cfl_store(f2 qmax, float scale, unsigned long long* to,
+                                                   unsigned slot) {
+    const float l = f2lo(qmax), h = f2hi(qmax);
+    float q = (h > l || h != h) ? h : l;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float v = __shfl_xor_sync(FULL, q, o);
+      q = (v > q || v != v) ? v : q;
+    }
+    if ((threadIdx.x & 31) == 0 && q != 0.0f)
+      atomicMax(to + slot % NSLOT, dkey((double)(q * scale)));
+  }
+
   // ------------------------------------------------------------ x sweep
 
   // predictor of one row; bd, bu: B_y of w at the rows below and above
@@ -325,7 +349,7 @@ struct Line2 {
 
   // rows gya .. gyb-1 (ghost-range indices)
   static __device__ void run_x(const FusedArgs& a, const Ctx& c, Pipe& pp, int gya, int gyb,
-                               f2& qmax) {
+                               f2& qmax, f2& qmax2) {
     // carried: w of rows r and r+1 (MHD); w1 and half slopes of row r; B_y
     // of w1 at row r-1 (MHD)
     f2 w0[NW], wp[NW], w1c[NW], hlc[NW];
@@ -374,8 +398,10 @@ struct Line2 {
         L[v] = w1c[v] + hlc[v];
         R[v] = f2m(rh, nb);
       }
-      const f2 cm = face(L, R, c.k, G);
+      f2 cm2;
+      const f2 cm = face(a, L, R, c.k, G, cm2);
       if (c.cfl) cfl_fold(cm, c.cflx, c.fv0, c.fv1, qmax);
+      if (ROE && c.cfl) cfl_fold(cm2, c.cflx, c.fv0, c.fv1, qmax2);
       // flux differences of the pair's cells
 #pragma unroll
       for (int v = 0; v < NW; v++) {
@@ -419,7 +445,7 @@ struct Line2 {
   // output rows gya .. gyb-1: iterations r = gya-1 .. gyb predict row r,
   // form the face (r-1|r) and update row r-1
   static __device__ void run_y(const FusedArgs& a, const Ctx& c, Pipe& pp, int gya, int gyb,
-                               f2& qmax) {
+                               f2& qmax, f2& qmax2) {
     f2 wm[NW], w0[NW], wp[NW], w1p[NW], hlp[NW], Gp[NW];
     f2 b1pp = f2s(0.0f);  // B_y of w1 at row r-2
     prime(c, pp, gya - 2);
@@ -467,8 +493,11 @@ struct Line2 {
         L[v] = w1p[v] + hlp[v];
         R[v] = w1[v] - hl[v];
       }
-      const f2 cm = face(L, R, c.k, G);
+      f2 cm2;
+      const f2 cm = face(a, L, R, c.k, G, cm2);
       if (c.cfl && r >= gya) cfl_fold(cm, f2s(2.0f / (dyp + dyc)), c.ok0, c.ok1, qmax);
+      if (ROE && c.cfl && r >= gya)
+        cfl_fold(cm2, f2s(2.0f / (dyp + dyc)), c.ok0, c.ok1, qmax2);
       // update of row r-1 (div B of its w1: the x part from the neighbour
       // lanes, formed by every lane before the branch)
       f2 db = f2s(0.0f);
@@ -563,27 +592,19 @@ struct Line2 {
     const int all = (1 << NW) - 1;
     c.fix_x = GEN && (c.bmx & 255) != all && (gxs <= 1 || gxs + 63 >= c.nX + 2);
     c.fix_y = GEN && (c.bmy & 255) != all;
-    f2 qmax = f2s(0.0f);
+    f2 qmax = f2s(0.0f), qmax2 = f2s(0.0f);
     Pipe pp;
     pp.sm = smem_u32(ring);
     pp.rd = (c.c0 - c.cs) * 4;
     if (D == 0)
-      run_x(a, c, pp, gya, gyb, qmax);
+      run_x(a, c, pp, gya, gyb, qmax, qmax2);
     else
-      run_y(a, c, pp, gya, gyb, qmax);
+      run_y(a, c, pp, gya, gyb, qmax, qmax2);
     drain();  // the ring's last copies land before the next item reuses it
     if (c.cfl) {
-      float q;
-      {
-        const float l = f2lo(qmax), h = f2hi(qmax);
-        q = (h > l || h != h) ? h : l;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float v = __shfl_xor_sync(FULL, q, o);
-        q = (v > q || v != v) ? v : q;
-      }
-      if (lane == 0 && q != 0.0f) atomicMax(&ctrl->face_cmax[D][slot % NSLOT], dkey((double)q));
+      // 'tvdmu' keeps |a|*dt*2/(dx+dx) of its two fast waves
+      cfl_store(qmax, ROE ? c.qdt : 1.0f, ctrl->face_cmax[D], slot);
+      if (ROE) cfl_store(qmax2, c.qdt, ctrl->face_cmax2[D], slot);
     }
   }
 };

@@ -4,23 +4,9 @@
 #include <cstring>
 
 #include "batch_items.cuh"
-#include "sweep_pair.cuh"
+#include "pair_launch.cuh"
 
 namespace vacgpu {
-
-template <int D, bool MHD, int LIMC, bool GEN>
-static void launch_pair_one(const CUtensorMap* map, const FusedArgs& a, dim3 grid,
-                            cudaStream_t st) {
-  constexpr int NW = MHD ? 8 : 5;
-  const int smem = pair_smem_floats(NW) * 4;
-  auto k = k_sweep_pair<D, MHD, LIMC, GEN>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    attr = true;
-  }
-  k<<<grid, PT_NT, smem, st>>>(*map, a);
-}
 
 // The grid needs the general form of the pair sweep (PairSweep's GEN):
 // gravity, a non-periodic face, split sources, no Powell terms for MHD, or
@@ -31,15 +17,6 @@ bool pair_general(const FusedArgs& a, bool mhd) {
              (mhd && !a.ph.divbfix);
   for (int d = 0; d < 3; d++) gen = gen || a.periodic_mask[d] != all;
   return gen;
-}
-
-template <int D, bool MHD, int LIMC>
-static void launch_pair_gen(const CUtensorMap* map, const FusedArgs& a, dim3 grid,
-                           cudaStream_t st) {
-  if (pair_general(a, MHD))
-    launch_pair_one<D, MHD, LIMC, true>(map, a, grid, st);
-  else
-    launch_pair_one<D, MHD, LIMC, false>(map, a, grid, st);
 }
 
 // VACGPU_PAIR=0 keeps the one-cell kernel for every grid (read once)
@@ -97,7 +74,9 @@ bool launch_sweep_pair(FusedArgs a, int D, bool mhd, const void* tmap, int nzc,
   a.nzc = nzc;
   dim3 grid(nxt, nyt, (a.g.nx[am] + nzc - 1) / nzc);
   const CUtensorMap* map = (const CUtensorMap*)tmap;
-#define LP(DD, M, L) launch_pair_gen<DD, M, L>(map, a, grid, st)
+  // the Roe instances are a unit of their own (roe_pair.cu)
+  if (a.ph.typefull == VACGPU_TVDMU) return launch_pair_roe(a, D, map, grid, st);
+#define LP(DD, M, L) launch_pair_gen<DD, M, L, false>(map, a, grid, st)
 #define LPD(DD)                                                              \
   if (D == DD) {                                                             \
     if (mhd) {                                                               \

@@ -35,6 +35,7 @@
 #include <cuda.h>
 
 #include "pack2.cuh"
+#include "roe_pair.cuh"
 #include "sweep_fused.cuh"
 
 namespace vacgpu {
@@ -232,8 +233,10 @@ __device__ __forceinline__ f2 p_hlim(f2 a, f2 b, const PairK& k) {
 // the general form (gravity, non-periodic faces, sources or the CFL
 // maximum switched off); false: the common case -- every face periodic,
 // unsplit sources with Powell's terms for MHD, no gravity, CFL maximum --
-// with those decisions fixed at compile time.
-template <int D, bool MHD, int LIMC, bool GEN>
+// with those decisions fixed at compile time.  ROE: the faces carry the Roe
+// dissipation of 'tvdmu' (MHD, no entropy fix) instead of TVDLF's, and the
+// CFL maximum is kept for its two fast waves.
+template <int D, bool MHD, int LIMC, bool GEN, bool ROE = false>
 struct PairSweep {
   static constexpr int K = D == 0 ? 0 : 2;        // in-plane / marching
   static constexpr int AM = D == 0 ? 2 : D;        // marching axis
@@ -308,12 +311,21 @@ struct PairSweep {
   }
 
   // TVDLF face flux 2F = F(L) + F(R) - cmax (R - L) and cmax of a pair of
-  // faces with left states L and right states R.
-  static __device__ __forceinline__ f2 face(const f2* L, const f2* R,
-                                            const PairK& k, f2* G) {
+  // faces with left states L and right states R (ROE: the Roe flux and
+  // |v + cf|, cm2 = |v - cf|).
+  static __device__ __forceinline__ f2 face(const FusedArgs& a, const f2* L, const f2* R,
+                                            const PairK& k, f2* G, f2& cm2) {
     f2 fL[NW], fR[NW], pL, pR, riL, riR;
     p_flux<D, MHD>(L, k, fL, pL, riL);
     p_flux<D, MHD>(R, k, fR, pR, riR);
+    if constexpr (ROE) {
+#pragma unroll
+      for (int v = 0; v < NW; v++) G[v] = fL[v] + fR[v];
+      f2 cm1;
+      p_roe_dissipation<D, 3>(L, R, pL, pR, riL, riR, k, f2s(a.ph.c2gf), a.ph.divbwave, G, cm1,
+                              cm2);
+      return cm1;
+    }
     f2 M[NW];
     M[0] = k.half * (L[0] + R[0]);
     M[1 + D] = k.half * (L[1 + D] + R[1 + D]);
@@ -376,12 +388,39 @@ struct PairSweep {
     return ((amask >> v) & 1) ? -src : src;
   }
 
+  // the running CFL maximum of a pair of faces (NaN kept)
+  static __device__ __forceinline__ void cfl_fold(f2 c, bool v0, bool v1, f2& qmax) {
+    float cl, ch, ql, qh;
+    f2u(c, cl, ch);
+    f2u(qmax, ql, qh);
+    if (v0) ql = (cl > ql || cl != cl) ? cl : ql;
+    if (v1) qh = (ch > qh || ch != ch) ? ch : qh;
+    qmax = f2m(ql, qh);
+  }
+  // the CTA's maximum of qmax into the slots of `to`
+  static __device__ __forceinline__ void cfl_store(f2 qmax, float scale, float* shq,
+                                                   unsigned long long* to, unsigned slotid) {
+    const float l = f2lo(qmax), h = f2hi(qmax);
+    float q = (h > l || h != h) ? h : l;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float v = __shfl_xor_sync(0xffffffffu, q, o);
+      q = (v > q || v != v) ? v : q;
+    }
+    if ((threadIdx.x & 31) == 0) shq[threadIdx.x >> 5] = q;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int i = 1; i < PT_NT / 32; i++) q = (shq[i] > q || shq[i] != shq[i]) ? shq[i] : q;
+      if (q != 0.0f) atomicMax(to + slotid % NSLOT, dkey((double)(q * scale)));
+    }
+  }
+
   static __device__ bool run(const CUtensorMap* map, const FusedArgs& a, float* sm,
                              int bx, int by, int bz, unsigned long long* bars,
                              int* uses, unsigned slotid) {
     Ctrl* ctrl = a.ctrl;
     if (ctrl->done) return true;
-    __shared__ float shq[PT_NT / 32];
+    __shared__ float shq[2][PT_NT / 32];
     const int tid = threadIdx.x;
     const DevGrid& g = a.g;
     const int nX = g.nx[0], nR = g.nx[AR], nM = g.nx[AM];
@@ -460,7 +499,7 @@ struct PairSweep {
     const long long sam = AM == 2 ? g.plane : g.P;
     const bool nearxr = gco[AR] < 4 || gco[AR] >= g.nx[AR] || gco[0] < 4 || gco[0] + 1 >= g.nx[0];
 
-    f2 qmax = f2s(0.0f);
+    f2 qmax = f2s(0.0f), qmax2 = f2s(0.0f);
     if (tid == 0) {
       issue(z0 - 2);
       issue(z0 - 1);
@@ -791,15 +830,12 @@ struct PairSweep {
             L[v] = w1p[v] + hlp[v];
             R[v] = w1[v] - hl_[v];
           }
-          const f2 cm = face(L, R, k, G);
+          f2 cm2;
+          const f2 cm = face(a, L, R, k, G, cm2);
           if (cfl) {
-            const float cf = 2.0f / (dxzp + dxzc);
-            float cl, ch, ql, qh;
-            f2u(cm * f2s(cf), cl, ch);
-            f2u(qmax, ql, qh);
-            if (ok0) ql = (cl > ql || cl != cl) ? cl : ql;
-            if (ok1) qh = (ch > qh || ch != ch) ? ch : qh;
-            qmax = f2m(ql, qh);
+            const f2 cf = f2s(2.0f / (dxzp + dxzc));
+            cfl_fold(cm * cf, ok0, ok1, qmax);
+            if (ROE) cfl_fold(cm2 * cf, ok0, ok1, qmax2);
           }
         }
       } else if (!edge) {
@@ -812,17 +848,14 @@ struct PairSweep {
           L[v] = w1[v] + hl_[v];
           R[v] = f2m(rh, nb);
         }
-        const f2 cm = face(L, R, k, G);
+        f2 cm2;
+        const f2 cm = face(a, L, R, k, G, cm2);
         if (cfl) {
           // faces (-1|0) .. (n-1|n) of mesh rows inside the chunk
-          float cl, ch, ql, qh;
-          f2u(cm * cflx, cl, ch);
-          f2u(qmax, ql, qh);
           const bool v0 = rowok && ix0 >= -1 && ix0 < nX;
           const bool v1 = rowok && ix0 + 1 >= -1 && ix0 + 1 < nX && hl < 15;
-          if (v0) ql = (cl > ql || cl != cl) ? cl : ql;
-          if (v1) qh = (ch > qh || ch != ch) ? ch : qh;
-          qmax = f2m(ql, qh);
+          cfl_fold(cm * cflx, v0, v1, qmax);
+          if (ROE) cfl_fold(cm2 * cflx, v0, v1, qmax2);
         }
         // flux differences of the pair's cells, and B_x(x+1)-B_x(x-1) of w1
 #pragma unroll
@@ -903,37 +936,23 @@ struct PairSweep {
       for (int s2 = 0; s2 < FWRING; s2++) uses[s2] += (np - s2 + FWRING - 1) / FWRING;
     }
     if (cfl) {
-      float q = fmaxf(f2lo(qmax), f2hi(qmax));
-      {
-        const float l = f2lo(qmax), h = f2hi(qmax);
-        q = (h > l || h != h) ? h : l;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float v = __shfl_xor_sync(0xffffffffu, q, o);
-        q = (v > q || v != v) ? v : q;
-      }
-      if ((tid & 31) == 0) shq[tid >> 5] = q;
-      __syncthreads();
-      if (tid == 0) {
-        for (int i = 1; i < PT_NT / 32; i++) q = (shq[i] > q || shq[i] != shq[i]) ? shq[i] : q;
-        const unsigned long long key = dkey((double)q);
-        if (q != 0.0f) atomicMax(&ctrl->face_cmax[D][slotid % NSLOT], key);
-      }
+      // 'tvdmu' keeps |a|*dt*2/(dx+dx) of its two fast waves
+      cfl_store(qmax, ROE ? qdt : 1.0f, shq[0], ctrl->face_cmax[D], slotid);
+      if (ROE) cfl_store(qmax2, qdt, shq[1], ctrl->face_cmax2[D], slotid);
     }
     return true;
   }
 };
 
-template <int D, bool MHD, int LIMC, bool GEN>
-__global__ void __launch_bounds__(PT_NT, 3)
+template <int D, bool MHD, int LIMC, bool GEN, bool ROE = false>
+__global__ void __launch_bounds__(PT_NT, ROE ? 2 : 3)
     k_sweep_pair(const __grid_constant__ CUtensorMap map, FusedArgs a) {
   extern __shared__ __align__(128) float dsm[];
   __shared__ __align__(8) unsigned long long bars[FWRING];
   init_bars(bars);
   int uses[FWRING] = {0, 0, 0, 0};
   const unsigned slotid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  PairSweep<D, MHD, LIMC, GEN>::run(&map, a, dsm, blockIdx.x, blockIdx.y, blockIdx.z, bars,
+  PairSweep<D, MHD, LIMC, GEN, ROE>::run(&map, a, dsm, blockIdx.x, blockIdx.y, blockIdx.z, bars,
                                    uses, slotid);
 }
 

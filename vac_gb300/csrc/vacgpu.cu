@@ -923,7 +923,7 @@ int vacgpu_internal_view(vacgpu_handle* h, HandleView* v) {
   for (int i = 0; i < 2; i++)
     for (int k = 0; k < 2; k++) v->tmap[i][k] = &h->tmap[i][k];
   v->nzc = h->nzc > 0 ? h->nzc : 32;  // a batch fills the GPU with its other grids
-  v->fused = h->fused;
+  v->fused = h->fused && h->p.typefull == VACGPU_TVDLF;
   return 0;
 }
 int vacgpu_internal_set_cur(vacgpu_handle* h, int cur) {
@@ -1192,7 +1192,9 @@ int vacgpu_create(const vacgpu_params* p, vacgpu_handle** out) {
   h->fused = p->precision == VACGPU_PREC_MIXED && p->dimsplit &&
              (p->ndim == 2 || p->ndim == 3) && p->ndir == p->ndim &&
              p->typelimited == VACGPU_LIMITED_ORIGINAL &&
-             p->typefull == VACGPU_TVDLF && !p->smallfix && !p->useprimitive &&
+             (p->typefull == VACGPU_TVDLF ||
+              fused_roe_applies(g, ph, p->ndir, p->physics == VACGPU_PHYS_MHD)) &&
+             !p->smallfix && !p->useprimitive &&
              !(p->physics == VACGPU_PHYS_MHD && p->eqpar[1] != 0.0);
   if (const char* fz = getenv("VACGPU_FUSED")) h->fused = h->fused && atoi(fz) != 0;
   // its ghost writes need uniform copy maps, periodic faces in pairs and

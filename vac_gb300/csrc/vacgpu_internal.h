@@ -301,6 +301,8 @@ void launch_correct_roe_mixed(const SweepArgs& s, const float* w,
 bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win,
                         float* wout,
                         const float* const* idxf, int nzc, cudaStream_t st);
+// the fused sweeps run this grid's 'tvdmu' (Roe) corrector
+bool fused_roe_applies(const DevGrid& g, const DevPhys& ph, int ndir, bool mhd);
 // rows of the fused sweep's TMA box: x and z sweeps and the 3-D y sweep
 // (k=0), the 2-D y sweep (k=1)
 constexpr int FUSED_BOX_ROWS[2] = {12, 10};
