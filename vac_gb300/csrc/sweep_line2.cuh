@@ -63,8 +63,7 @@ struct Line2 {
   static constexpr int HALO = (D == 0 || MHD) ? 2 : 0;
   static constexpr int TW = 64 - 2 * HALO;     // output columns per strip
   static constexpr unsigned FULL = 0xffffffffu;
-  typedef PairSweep<2, MHD, LIMC, GEN> PS;     // for gfix
-  typedef Fused<3, 0, true, PREC_FF, LIMC_MINMOD> FX;  // for preimages
+  typedef PairSweep<2, MHD, LIMC, GEN> PS;     // for gfix, preimages and flip
 
   // Per-warp constants of a work item.
   struct Ctx {
@@ -249,25 +248,52 @@ struct Line2 {
     if (c.srcs) sources(a, c, c.qs1, u, c.nqs1h * divb, w1);
   }
 
-  // getboundary's ghost images of one new cell value (gx, gy) (one lane):
-  // the composition of the region copies of src/vacgrid.t:195-413
-  static __device__ __forceinline__ void ghost_images(const FusedArgs& a, const Ctx& c,
-                                                      int gx, int gy, const float* s) {
-    int x1, x2, fx, y1, y2, fy;
-    const int nx_ = 1 + FX::preimages(a, 0, gx, x1, fx, x2);
-    const int ny_ = 1 + FX::preimages(a, 1, gy, y1, fy, y2);
+  // Preimages of the index gi along axis d, as PairSweep's
+  static __device__ __forceinline__ int preimages(const FusedArgs& a, int d, int gi, int& p1,
+                                                  int& f1, int& p2) {
+    return PS::preimages(a, d, gi, p1, f1, p2);
+  }
+
+  // getboundary's ghost images of the pair at row gy, as PairSweep::images:
+  // images along y as pairs, those along x cell by cell
+  static __device__ __forceinline__ void images(const FusedArgs& a, const Ctx& c, int gy,
+                                                const f2* acc) {
+    int r1, r2, fr, x1, x2, fx, y1, y2, fy;
+    const int nr = 1 + preimages(a, 1, gy, r1, fr, r2);
+    const int na = c.ok0 ? preimages(a, 0, c.c0, x1, fx, x2) : 0;
+    const int nb = c.ok1 ? preimages(a, 0, c.c0 + 1, y1, fy, y2) : 0;
 #pragma unroll 1
-    for (int jj = 0; jj < ny_; jj++) {
-      const int py = jj == 0 ? gy : (jj == 1 ? y1 : y2);
-      const int sy = jj == 1 ? fy : 0;
-#pragma unroll 1
-      for (int i = 0; i < nx_; i++) {
-        if ((i | jj) == 0) continue;
-        const int px = i == 0 ? gx : (i == 1 ? x1 : x2);
-        const int fl = (i == 1 ? fx : 0) ^ sy;
-        float* o = c.wout + (long long)py * c.P + px;
+    for (int j = 0; j < nr; j++) {
+      const int pr = j == 0 ? gy : (j == 1 ? r1 : r2);
+      const int fl = j == 1 ? fr : 0;
+      float* o = c.wout + (long long)pr * c.P + c.c0;
+      if (j) {
 #pragma unroll
-        for (int v = 0; v < NW; v++) o[v * c.vs] = ((fl >> v) & 1) ? -s[v] : s[v];
+        for (int v = 0; v < NW; v++) {
+          const f2 s = PS::flip(acc[v], fl, v);
+          if (c.ok0 && c.ok1) {
+            st2(o + v * c.vs, s);
+          } else {
+            if (c.ok0) o[v * c.vs] = f2lo(s);
+            if (c.ok1) o[1 + v * c.vs] = f2hi(s);
+          }
+        }
+      }
+      if (na | nb) {
+#pragma unroll 1
+        for (int i = 1; i <= na; i++) {
+          float* q = o + ((i == 1 ? x1 : x2) - c.c0);
+          const int f = fl ^ (i == 1 ? fx : 0);
+#pragma unroll
+          for (int v = 0; v < NW; v++) q[v * c.vs] = f2lo(PS::flip(acc[v], f, v));
+        }
+#pragma unroll 1
+        for (int i = 1; i <= nb; i++) {
+          float* q = o + ((i == 1 ? y1 : y2) - c.c0);
+          const int f = fl ^ (i == 1 ? fy : 0);
+#pragma unroll
+          for (int v = 0; v < NW; v++) q[v * c.vs] = f2hi(PS::flip(acc[v], f, v));
+        }
       }
     }
   }
@@ -288,17 +314,7 @@ struct Line2 {
         if (c.ok1) o[1 + v * c.vs] = hi;
       }
     }
-    const bool neary = gy < 4 || gy >= c.nY;
-    if (!(neary || c.c0 < 4 || c.c0 + 1 >= c.nX)) return;
-#pragma unroll 1
-    for (int h = 0; h < 2; h++) {
-      const int gx = c.c0 + h;
-      if (!(h ? c.ok1 : c.ok0) || !(neary || gx < 4 || gx >= c.nX)) continue;
-      float s[NW];
-#pragma unroll
-      for (int v = 0; v < NW; v++) s[v] = h ? f2hi(acc[v]) : f2lo(acc[v]);
-      ghost_images(a, c, gx, gy, s);
-    }
+    if (gy < 4 || gy >= c.nY || c.c0 < 4 || c.c0 + 1 >= c.nX) images(a, c, gy, acc);
   }
 
   static __device__ __forceinline__ void cfl_fold(f2 cm, f2 cf, bool v0, bool v1, f2& qmax) {

@@ -359,24 +359,82 @@ struct PairSweep {
         if (ok1) a.wout[off + 1 + v * g.vs] = hi;
       }
     }
-    if (!(nearxr || gm < 4 || gm >= g.nx[AM])) return;
-    int gc[3];
-    gc[0] = gx;
-    gc[AR] = gr;
-    gc[AM] = gm;
-#pragma unroll 1
-    for (int h = 0; h < 2; h++) {
-      if (!(h ? ok1 : ok0)) continue;
-      int c2[3] = {gc[0] + h, gc[1], gc[2]};
-      bool near = false;
-#pragma unroll
-      for (int d = 0; d < 3; d++) near = near || c2[d] < 4 || c2[d] >= g.nx[d];
-      if (!near) continue;
-      float s[NW];
-#pragma unroll
-      for (int v = 0; v < NW; v++) s[v] = h ? f2hi(acc[v]) : f2lo(acc[v]);
-      write_ghost_images<3, NW>(a.g, a.ph, a.wout, c2, off + h, s);
+    if (nearxr || gm < 4 || gm >= g.nx[AM]) images(a, acc, off, gx, gr, gm, ok0, ok1);
+  }
+
+  // Preimages of the index gi along axis d (ghost_preimages; with every face
+  // periodic its one case).
+  static __device__ __forceinline__ int preimages(const FusedArgs& a, int d, int gi, int& p1,
+                                                  int& f1, int& p2) {
+    if constexpr (GEN) {
+      return ghost_preimages(a.g, a.ph, d, gi, p1, f1, p2);
+    } else {
+      const int n = a.g.nx[d];
+      p1 = p2 = gi < 4 ? gi + n : gi - n;
+      f1 = 0;
+      return gi < 4 || gi >= n;
     }
+  }
+
+  // The ghost images of a pair (ghost_images.cuh).  Images along the row and
+  // the marching axis shift both cells alike and go out as pairs; only the
+  // two or three columns beside an x face store their cells one by one.  (One
+  // cell at a time made a CTA at a face take up to twice an interior one's
+  // time, 187 us against 101 at 192^3.  MHD sweeps on periodic grids with it
+  // and without: 256^3 512 us against 574, 127^3 96 against 114, 64^3 27
+  // against 33; 2-D, 1001^2 40 against 46, 128^2 11 against 12.)
+  static __device__ __forceinline__ void images(const FusedArgs& a, const f2* acc, long long off,
+                                                int gx, int gr, int gm, bool ok0, bool ok1) {
+    const DevGrid& g = a.g;
+    int r1, r2, fr, m1, m2, fm, x1, x2, fx, y1, y2, fy;
+    const int nr = 1 + preimages(a, AR, gr, r1, fr, r2);
+    const int nm = 1 + preimages(a, AM, gm, m1, fm, m2);
+    const int na = ok0 ? preimages(a, 0, gx, x1, fx, x2) : 0;
+    const int nb = ok1 ? preimages(a, 0, gx + 1, y1, fy, y2) : 0;
+    const long long sr = AR == 2 ? g.plane : g.P, sm = AM == 2 ? g.plane : g.P;
+#pragma unroll 1
+    for (int k = 0; k < nm; k++) {
+      const int pm = k == 0 ? gm : (k == 1 ? m1 : m2);
+#pragma unroll 1
+      for (int j = 0; j < nr; j++) {
+        const int pr = j == 0 ? gr : (j == 1 ? r1 : r2);
+        const int fl = (k == 1 ? fm : 0) ^ (j == 1 ? fr : 0);
+        float* o = a.wout + off + (pm - gm) * sm + (pr - gr) * sr;
+        if (k | j) {
+#pragma unroll
+          for (int v = 0; v < NW; v++) {
+            const f2 s = flip(acc[v], fl, v);
+            if (ok0 && ok1) {
+              st2(o + v * g.vs, s);
+            } else {
+              if (ok0) o[v * g.vs] = f2lo(s);
+              if (ok1) o[1 + v * g.vs] = f2hi(s);
+            }
+          }
+        }
+        if (na | nb) {
+#pragma unroll 1
+          for (int i = 1; i <= na; i++) {
+            float* q = o + ((i == 1 ? x1 : x2) - gx);
+            const int f = fl ^ (i == 1 ? fx : 0);
+#pragma unroll
+            for (int v = 0; v < NW; v++) q[v * g.vs] = f2lo(flip(acc[v], f, v));
+          }
+#pragma unroll 1
+          for (int i = 1; i <= nb; i++) {
+            float* q = o + ((i == 1 ? y1 : y2) - gx);
+            const int f = fl ^ (i == 1 ? fy : 0);
+#pragma unroll
+            for (int v = 0; v < NW; v++) q[v * g.vs] = f2hi(flip(acc[v], f, v));
+          }
+        }
+      }
+    }
+  }
+  // acc, negated where bit v of fl is set ('asymm' faces: the general form)
+  static __device__ __forceinline__ f2 flip(f2 acc, int fl, int v) {
+    if constexpr (GEN) acc.v ^= ((fl >> v) & 1) ? 0x8000000080000000ull : 0ull;
+    return acc;
   }
 
   // per-variable ghost fix of a predictor value (getboundary on w1 at a
