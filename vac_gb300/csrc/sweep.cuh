@@ -1178,8 +1178,9 @@ struct Launch {
     VACGPU_DISPATCH(a, KC);
 #undef KC
   }
-  static void ghost(const SweepArgs& a, T* w, cudaStream_t st) {
-    long long n = ghost_count(a.g);
+  // yz: the y and z layers alone (ghost_cell counts the x layers last)
+  static void ghost(const SweepArgs& a, T* w, cudaStream_t st, bool yz = false) {
+    long long n = ghost_count(a.g) - (yz ? 4LL * a.g.nx[1] * a.g.nx[2] : 0);
     unsigned nb = grid_for(n, 128);
     int nw = a.mhd ? 2 + 2 * a.ndir : 2 + a.ndir;
     switch (nw) {
@@ -1298,6 +1299,9 @@ struct Launch {
   }                                                                          \
   void launch_ghost_##SUF(const SweepArgs& s, PH::T* w, cudaStream_t st) {   \
     Launch<PH>::ghost(s, w, st);                                             \
+  }                                                                          \
+  void launch_ghost_yz_##SUF(const SweepArgs& s, PH::T* w, cudaStream_t st) { \
+    Launch<PH>::ghost(s, w, st, true);                                       \
   }                                                                          \
   void launch_source_pass_##SUF(const SweepArgs& s, const PH::T* wct,        \
                                 PH::T* w, int pred, cudaStream_t st) {       \

@@ -62,6 +62,7 @@ static void launch_one(const CUtensorMap* map, const FusedArgs& a, dim3 grid,
 }
 
 bool pair_applies(const FusedArgs& a, bool mhd);
+bool pair_general(const FusedArgs& a, bool mhd);
 bool line2_applies(const FusedArgs& a, bool mhd);
 
 // The fused sweeps with the Roe dissipation of 'tvdmu': ideal MHD without an
@@ -107,8 +108,10 @@ bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win, 
     }
   // 3-D grids: the two-cells-per-thread kernel (packed FP32) where it
   // applies; VACGPU_PAIR=0 keeps the one-cell kernel
-  if (nd == 3 && launch_sweep_pair(a, s.d0, s.mhd, tmap, nzc, st))
+  if (nd == 3 && launch_sweep_pair(a, s.d0, s.mhd, tmap, nzc, st)) {
+    if (pair_general(a, s.mhd)) launch_ghost_yz_mixed(s, wout, st);
     return true;
+  }
   // 2-D grids: the warp-marching two-cells-per-thread kernel where it applies
   if (nd == 2 && launch_sweep_line2(a, win, s.d0, s.mhd, st)) return true;
   // the one-cell kernel: tiles over x and the row axis, z chunks along the

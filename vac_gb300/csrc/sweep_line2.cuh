@@ -63,7 +63,7 @@ struct Line2 {
   static constexpr int HALO = (D == 0 || MHD) ? 2 : 0;
   static constexpr int TW = 64 - 2 * HALO;     // output columns per strip
   static constexpr unsigned FULL = 0xffffffffu;
-  typedef PairSweep<2, MHD, LIMC, GEN> PS;     // for gfix, preimages and flip
+  typedef PairSweep<2, MHD, LIMC, GEN> PS;     // for preimages and flip
 
   // Per-warp constants of a work item.
   struct Ctx {
@@ -150,6 +150,14 @@ struct Line2 {
     asm volatile("cp.async.wait_all;" ::: "memory");
   }
 
+  // per-variable ghost fix of a predictor value (getboundary on w1 at a
+  // non-periodic face): src for the variables not periodic in that
+  // dimension, negated where 'asymm'
+  static __device__ __forceinline__ float gfix(float own, float src, int v, int pmask,
+                                               int amask) {
+    if ((pmask >> v) & 1) return own;
+    return ((amask >> v) & 1) ? -src : src;
+  }
   // getboundary of w1 at the x faces of a strip that reaches them: the
   // first ghost column takes the adjacent mesh value (non-periodic
   // variables, negated where 'asymm')
@@ -161,9 +169,9 @@ struct Line2 {
       const float dn = __shfl_down_sync(FULL, lo, 1);
       const float up = __shfl_up_sync(FULL, hi, 1);
       const int pm = c.bmx & 255, al = (c.bmx >> 8) & 255, ah = c.bmx >> 16;
-      if (c.c0 + 1 == 1) hi = PS::gfix(hi, dn, v, pm, al);
-      if (c.c0 == c.nX + 2) lo = PS::gfix(lo, up, v, pm, ah);
-      if (c.c0 + 1 == c.nX + 2) hi = PS::gfix(hi, lo, v, pm, ah);
+      if (c.c0 + 1 == 1) hi = gfix(hi, dn, v, pm, al);
+      if (c.c0 == c.nX + 2) lo = gfix(lo, up, v, pm, ah);
+      if (c.c0 + 1 == c.nX + 2) hi = gfix(hi, lo, v, pm, ah);
       w1[v] = f2m(lo, hi);
     }
   }
@@ -173,7 +181,7 @@ struct Line2 {
     float ol, oh, sl, sh;
     f2u(own, ol, oh);
     f2u(src, sl, sh);
-    return f2m(PS::gfix(ol, sl, v, c.bmy & 255, amask), PS::gfix(oh, sh, v, c.bmy & 255, amask));
+    return f2m(gfix(ol, sl, v, c.bmy & 255, amask), gfix(oh, sh, v, c.bmy & 255, amask));
   }
 
   // addsource2 with wCT = wc: gravity, then Powell's terms for

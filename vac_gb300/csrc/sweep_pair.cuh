@@ -236,7 +236,13 @@ __device__ __forceinline__ f2 p_hlim(f2 a, f2 b, const PairK& k) {
 // with those decisions fixed at compile time.  ROE: the faces carry the Roe
 // dissipation of 'tvdmu' (MHD, no entropy fix) instead of TVDLF's, and the
 // CFL maximum is kept for its two fast waves.
-template <int D, bool MHD, int LIMC, bool GEN, bool ROE = false>
+// IMG: the sweep writes all ghost images of its output; otherwise those at
+// the x faces, and the caller fills the y and z layers.  The loops over the
+// images of the general index maps make the CTAs at a face, and with them the
+// sweep, slower than a fill of the y and z layers behind it (9 us at 128^3, 11
+// at 192^3) -- with outflow faces 128^3 took 129 us, 112 now -- so single
+// grids leave them out; a batch, which has no fill, keeps them.
+template <int D, bool MHD, int LIMC, bool GEN, bool ROE = false, bool IMG = true>
 struct PairSweep {
   static constexpr int K = D == 0 ? 0 : 2;        // in-plane / marching
   static constexpr int AM = D == 0 ? 2 : D;        // marching axis
@@ -253,6 +259,23 @@ struct PairSweep {
   // transverse B of the predictor: component c (0: B_x, 1: B_AR) of plane p
   static __device__ __forceinline__ float* wb(float* sm, int p, int c, int ly, int lx) {
     return sm + FWRING * SLOT + ((p & 1) * 2 + c) * WBC + (ly + 1) * WBP + lx + WBO;
+  }
+
+  // w, negated where variable v is 'asymm' (bit v of amask): the predictor at
+  // a ghost position beside a non-periodic face, from the adjacent mesh value
+  // w (getboundary on w1).  (A fused grid's faces have one map for every
+  // variable, so a face is periodic for all of them or for none.)
+  static __device__ __forceinline__ f2 wflip(f2 w, int v, int amask) {
+    w.v ^= ((amask >> v) & 1) ? 0x8000000080000000ull : 0ull;
+    return w;
+  }
+  // the predictor's B_AR of a pair at tile row ly, and of the ghost row that
+  // takes it at a non-periodic row face (rlo, rhi; re: local row nR)
+  static __device__ __forceinline__ void store_br(const FusedArgs& a, float* sm, int j, int ly,
+                                                  int lx0, f2 w, bool rlo, bool rhi, int re) {
+    if (!(rhi && ly >= re)) st2(wb(sm, j, 1, ly, lx0), w);
+    if (rlo && ly == 0) st2(wb(sm, j, 1, -1, lx0), wflip(w, 5 + AR, a.asymm_lo[AR]));
+    if (rhi && ly == re - 1) st2(wb(sm, j, 1, re, lx0), wflip(w, 5 + AR, a.asymm_hi[AR]));
   }
 
   // Hancock predictor of the magnetic component B_k alone at a pair of
@@ -359,7 +382,11 @@ struct PairSweep {
         if (ok1) a.wout[off + 1 + v * g.vs] = hi;
       }
     }
-    if (nearxr || gm < 4 || gm >= g.nx[AM]) images(a, acc, off, gx, gr, gm, ok0, ok1);
+    if constexpr (IMG) {
+      if (nearxr || gm < 4 || gm >= g.nx[AM]) images(a, acc, off, gx, gr, gm, ok0, ok1);
+    } else {
+      if (gx < 4 || gx + 1 >= g.nx[0]) ximages(a, acc, off, gx, ok0, ok1);
+    }
   }
 
   // Preimages of the index gi along axis d (ghost_preimages; with every face
@@ -431,19 +458,48 @@ struct PairSweep {
       }
     }
   }
+  // The ghost images of a pair at the x faces alone.  The pair beside a face
+  // stores its two, which lie side by side, at once where they start on an
+  // even column; cells of a pair that the mesh or the tile cuts go one by one.
+  static __device__ __forceinline__ void ximages(const FusedArgs& a, const f2* acc,
+                                                 long long off, int gx, bool ok0, bool ok1) {
+    const DevGrid& g = a.g;
+    const int n = g.nx[0];
+    const bool lo = gx < 4;
+    const int m = a.ph.gmap[0][lo ? 0 : 1], fl = m == GMAP_MIRROR ? a.ph.asym[0][lo ? 0 : 1] : 0;
+    float* o = a.wout + off;
+    if (ok0 && ok1 && (lo || gx == n) && !(m == GMAP_PERIODIC && (n & 1))) {
+      const int d = m == GMAP_PERIODIC ? (lo ? n : -n) : (lo ? -2 : 2);
+#pragma unroll
+      for (int v = 0; v < NW; v++) {
+        const f2 s = flip(acc[v], fl, v);
+        const float l = f2lo(s), h = f2hi(s);
+        st2(o + d + v * g.vs, m == GMAP_PERIODIC ? s : m == GMAP_MIRROR ? f2m(h, l)
+                                                       : lo ? f2m(l, l) : f2m(h, h));
+      }
+      return;
+    }
+#pragma unroll 1
+    for (int c = 0; c < 2; c++) {
+      if (!(c ? ok1 : ok0)) continue;
+      int p1, p2, f1;
+      const int k = ghost_preimages(g, a.ph, 0, gx + c, p1, f1, p2);
+#pragma unroll 1
+      for (int i = 0; i < k; i++) {
+        float* q = o + ((i ? p2 : p1) - gx);
+#pragma unroll
+        for (int v = 0; v < NW; v++) {
+          const f2 s = flip(acc[v], i ? 0 : f1, v);
+          q[v * g.vs] = c ? f2hi(s) : f2lo(s);
+        }
+      }
+    }
+  }
+
   // acc, negated where bit v of fl is set ('asymm' faces: the general form)
   static __device__ __forceinline__ f2 flip(f2 acc, int fl, int v) {
     if constexpr (GEN) acc.v ^= ((fl >> v) & 1) ? 0x8000000080000000ull : 0ull;
     return acc;
-  }
-
-  // per-variable ghost fix of a predictor value (getboundary on w1 at a
-  // non-periodic face): src for the variables not periodic in that
-  // dimension, negated where 'asymm'
-  static __device__ __forceinline__ float gfix(float own, float src, int v, int pmask,
-                                               int amask) {
-    if ((pmask >> v) & 1) return own;
-    return ((amask >> v) & 1) ? -src : src;
   }
 
   // the running CFL maximum of a pair of faces (NaN kept)
@@ -544,7 +600,17 @@ struct PairSweep {
                  2.0f / (a.dxf[0][gx1] + a.dxf[0][min(ix0 + 4, g.nG[0] - 1)]));
     // ghost fixes of the predictor at non-periodic faces
     const bool fix_x = GEN && a.periodic_mask[0] != all && (x0 <= 0 || x0 + TX + 1 >= nX);
-    const bool fix_r = GEN && a.periodic_mask[AR] != all && (y0 == 0 || y0 + TY >= nR);
+    // transverse B of the predictor beside a non-periodic x or row face: the
+    // ghost columns (local -1 or xe) and rows (-1 or re) take the adjacent
+    // mesh value, which the thread that owns it stores there; the threads and
+    // warps that would predict them store nothing.  (A pass over the planes in
+    // shared memory behind a second barrier did this before, at 8 % of a 256^3
+    // sweep with outflow faces.)
+    const bool npx = GEN && K == 2 && !((a.periodic_mask[0] >> 5) & 1);
+    const bool npr = GEN && !((a.periodic_mask[AR] >> (5 + AR)) & 1);
+    const int xe = nX - x0, re = nR - y0;
+    const bool xlo = npx && x0 == 0, xhi = npx && xe <= TX;
+    const bool rlo = npr && y0 == 0, rhi = npr && re <= TY;
     const bool fix_m = GEN && a.periodic_mask[AM] != all;
     // the pair's output offset at marching-axis ghost index 0, the stride
     // along that axis, and whether it lies within two cells of an x or
@@ -647,36 +713,27 @@ struct PairSweep {
         // marching-axis ghost planes: w1(-1) from w1(0), w1(n) from w1(n-1)
         if (fix_m && j == 0) {
 #pragma unroll
-          for (int v = 0; v < NW; v++) {
-            float ol, oh, sl, sh2;
-            f2u(w1p[v], ol, oh);
-            f2u(w1[v], sl, sh2);
-            w1p[v] = f2m(gfix(ol, sl, v, a.periodic_mask[AM], a.asymm_lo[AM]),
-                         gfix(oh, sh2, v, a.periodic_mask[AM], a.asymm_lo[AM]));
-          }
+          for (int v = 0; v < NW; v++) w1p[v] = wflip(w1[v], v, a.asymm_lo[AM]);
           bzm1 = w1p[5 + AM];
         }
         if (fix_m && j == nM) {
 #pragma unroll
-          for (int v = 0; v < NW; v++) {
-            float ol, oh, sl, sh2;
-            f2u(w1[v], ol, oh);
-            f2u(w1p[v], sl, sh2);
-            w1[v] = f2m(gfix(ol, sl, v, a.periodic_mask[AM], a.asymm_hi[AM]),
-                        gfix(oh, sh2, v, a.periodic_mask[AM], a.asymm_hi[AM]));
-          }
+          for (int v = 0; v < NW; v++) w1[v] = wflip(w1p[v], v, a.asymm_hi[AM]);
         }
         // an odd mesh width: the first ghost column is the second cell of the
         // last pair, whose B_x the first cell's div B takes from registers
         if (fix_x && ix0 + 1 == nX) {
-          float lo, hi;
-          f2u(w1[5], lo, hi);
-          w1[5] = f2m(lo, gfix(hi, lo, 5, a.periodic_mask[0], a.asymm_hi[0]));
+          const float lo = f2lo(w1[5]);
+          w1[5] = f2m(lo, f2lo(wflip(w1[5], 5, a.asymm_hi[0])));
         }
         bz = w1[5 + AM];
         if (ring) {
-          st2(wb(sm, j, 0, ly, lx0), w1[5]);
-          st2(wb(sm, j, 1, ly, lx0), w1[5 + AR]);
+          if (!(xhi && lx0 >= xe)) st2(wb(sm, j, 0, ly, lx0), w1[5]);
+          if (xlo && lx0 == 0)
+            *wb(sm, j, 0, ly, -1) = f2lo(wflip(w1[5], 5, a.asymm_lo[0]));
+          if (xhi && lx0 + 2 == xe)
+            *wb(sm, j, 0, ly, xe) = f2hi(wflip(w1[5], 5, a.asymm_hi[0]));
+          store_br(a, sm, j, ly, lx0, w1[5 + AR], rlo, rhi, re);
           // transverse B of the ring: rows -1 and TY (warp 0, B_AR), columns
           // -1 and TX (warp 1, lanes 0-7, B_x)
           const int wq = tid >> 5;
@@ -717,10 +774,10 @@ struct PairSweep {
             const f2 divb = ffma(dbz, idxz, ffma(dby, iy_, dbx * ix_));
             const f2 o = predict_b(c, cp, cm_, qdt2 * idxz, nqs1h * divb, true, k);
             if (wq == 0) {
-              st2(wb(sm, j, 1, rl, lx0), o);
+              if (!(rl < 0 ? rlo : rhi)) st2(wb(sm, j, 1, rl, lx0), o);
             } else {
-              *wb(sm, j, 0, rl, -1) = f2lo(o);
-              *wb(sm, j, 0, rl, TX) = f2hi(o);
+              if (!xlo) *wb(sm, j, 0, rl, -1) = f2lo(o);
+              if (!xhi) *wb(sm, j, 0, rl, TX) = f2hi(o);
             }
           }
         }
@@ -786,25 +843,34 @@ struct PairSweep {
           }
           // x-face ghost cells of the region: w1(-1) from w1(0), w1(n) from
           // w1(n-1) (the pair's first cell has an even index)
-          if (fix_x) {
+          if (fix_x && x0 < 0) {
 #pragma unroll
             for (int v = 0; v < NW; v++) {
-              float lo, hi;
-              f2u(w1[v], lo, hi);
-              const float dn = __shfl_down_sync(0xffffffffu, lo, 1, 16);
-              const float upv = __shfl_up_sync(0xffffffffu, hi, 1, 16);
-              const int pmk = a.periodic_mask[0];
-              if (ix0 + 1 == -1) hi = gfix(hi, dn, v, pmk, a.asymm_lo[0]);
-              if (ix0 == nX) lo = gfix(lo, upv, v, pmk, a.asymm_hi[0]);
-              if (ix0 + 1 == nX) hi = gfix(hi, lo, v, pmk, a.asymm_hi[0]);
-              w1[v] = f2m(lo, hi);
+              const float dn =
+                  __shfl_down_sync(0xffffffffu, f2lo(wflip(w1[v], v, a.asymm_lo[0])), 1, 16);
+              if (ix0 == -2) w1[v] = f2m(f2lo(w1[v]), dn);
+            }
+          }
+          if (fix_x && x0 + TX + 1 >= nX) {
+            if (nX & 1) {
+#pragma unroll
+              for (int v = 0; v < NW; v++)
+                if (ix0 + 1 == nX)
+                  w1[v] = f2m(f2lo(w1[v]), f2lo(wflip(w1[v], v, a.asymm_hi[0])));
+            } else {
+#pragma unroll
+              for (int v = 0; v < NW; v++) {
+                const float up =
+                    __shfl_up_sync(0xffffffffu, f2hi(wflip(w1[v], v, a.asymm_hi[0])), 1, 16);
+                if (ix0 == nX) w1[v] = f2m(up, f2hi(w1[v]));
+              }
             }
           }
           bz = w1[5 + AM];
 #pragma unroll
           for (int v = 0; v < NW; v++) hl_[v] = hlv[v];
           if (ring) {
-            st2(wb(sm, j, 1, ly, lx0), w1[5 + AR]);
+            store_br(a, sm, j, ly, lx0, w1[5 + AR], rlo, rhi, re);
             if ((tid >> 5) == 0) {
               // B_y of the ring rows -1 and TY
               const int rr = lane < 16 ? 1 : TY + 2;
@@ -826,56 +892,15 @@ struct PairSweep {
               const f2 dbz = ld2(pp + (5 + AM) * BPL + ob) - ld2(pm + (5 + AM) * BPL + ob);
               const f2 iy_ = f2s(a.idxf[AR][min(max(y0 + rl + 2, 0), g.nG[AR] - 1)]);
               const f2 divb = ffma(dbz, idxz, ffma(dby, iy_, dbx2 * idxx));
-              st2(wb(sm, j, 1, rl, lx0), predict_b(c, cp, cm_, qdt2 * idxx, nqs1h * divb, true, k));
+              const f2 o = predict_b(c, cp, cm_, qdt2 * idxx, nqs1h * divb, true, k);
+              if (!(rl < 0 ? rlo : rhi)) st2(wb(sm, j, 1, rl, lx0), o);
             }
           }
         }
         // marching-axis ghost planes of B_AM
-        if (fix_m && j == 0) {
-          float ol, oh, sl, sh2;
-          f2u(bzm1, ol, oh);
-          f2u(bz, sl, sh2);
-          bzm1 = f2m(gfix(ol, sl, 5 + AM, a.periodic_mask[AM], a.asymm_lo[AM]),
-                     gfix(oh, sh2, 5 + AM, a.periodic_mask[AM], a.asymm_lo[AM]));
-        }
-        if (fix_m && j == nM) {
-          float ol, oh, sl, sh2;
-          f2u(bz, ol, oh);
-          f2u(bzm1, sl, sh2);
-          bz = f2m(gfix(ol, sl, 5 + AM, a.periodic_mask[AM], a.asymm_hi[AM]),
-                   gfix(oh, sh2, 5 + AM, a.periodic_mask[AM], a.asymm_hi[AM]));
-        }
+        if (fix_m && j == 0) bzm1 = wflip(bz, 5 + AM, a.asymm_lo[AM]);
+        if (fix_m && j == nM) bz = wflip(bzm1, 5 + AM, a.asymm_hi[AM]);
       }
-      // getboundary of the ring/tile predictor values at non-periodic x and
-      // row faces (read at the next iteration's update).  The transverse B
-      // of plane j in w1b is otherwise read only at the next iteration,
-      // after its barrier A, so this barrier is needed only here.
-      if (ring && (fix_r || (K == 2 && fix_x))) {
-        __syncthreads();  // barrier B: w1b of plane j complete
-        for (int c = tid; c < 36 * 10; c += PT_NT) {
-          const int lx = c % 36 - WBO, lyy = c / 36 - 1;
-          const int ixc = x0 + lx, iyc = y0 + lyy;
-          int d = -1, slx = lx, sly = lyy, lo = 0;
-          if (K == 2 && (ixc == -1 || ixc == nX) && iyc >= 0 && iyc < nR) {
-            d = 0;
-            lo = ixc == -1;
-            slx = lx + (lo ? 1 : -1);
-          } else if ((iyc == -1 || iyc == nR) && ixc >= 0 && ixc < nX) {
-            d = AR;
-            lo = iyc == -1;
-            sly = lyy + (lo ? 1 : -1);
-          }
-          if (d < 0) continue;
-          const int asy = lo ? a.asymm_lo[d] : a.asymm_hi[d];
-#pragma unroll
-          for (int cc = K == 2 ? 0 : 1; cc < 2; cc++) {
-            const int v = cc == 0 ? 5 : 5 + AR;
-            float* dst = wb(sm, j, cc, lyy, lx);
-            *dst = gfix(*dst, *wb(sm, j, cc, sly, slx), v, a.periodic_mask[d], asy);
-          }
-        }
-      }
-
       // ---------------- faces of plane j (in-plane) or between j-1 and j
       f2 G[NW];
 #pragma unroll
@@ -1010,8 +1035,8 @@ __global__ void __launch_bounds__(PT_NT, ROE ? 2 : 3)
   init_bars(bars);
   int uses[FWRING] = {0, 0, 0, 0};
   const unsigned slotid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  PairSweep<D, MHD, LIMC, GEN, ROE>::run(&map, a, dsm, blockIdx.x, blockIdx.y, blockIdx.z, bars,
-                                   uses, slotid);
+  PairSweep<D, MHD, LIMC, GEN, ROE, !GEN>::run(&map, a, dsm, blockIdx.x, blockIdx.y, blockIdx.z,
+                                               bars, uses, slotid);
 }
 
 }  // namespace vacgpu

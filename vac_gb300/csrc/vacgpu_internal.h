@@ -264,6 +264,7 @@ struct SweepArgs {
   void launch_correct_##SUF(const SweepArgs& s, const T* w, const T* w1,     \
                             const T* base, T* wout, cudaStream_t st);        \
   void launch_ghost_##SUF(const SweepArgs& s, T* w, cudaStream_t st);        \
+  void launch_ghost_yz_##SUF(const SweepArgs& s, T* w, cudaStream_t st);     \
   void launch_source_pass_##SUF(const SweepArgs& s, const T* wct, T* w,     \
                                 int pred, cudaStream_t st);                  \
   void launch_pminmax_##SUF(const SweepArgs& s, const T* w, cudaStream_t st); \
