@@ -247,7 +247,7 @@ def _physical(w, gamma, mhd):
 
 def _fresh_timed(params, snap, k, stream, warm):
     """A new engine on the seeded state: `warm` untimed steps (graph capture,
-    z-chunk tuning), the state uploaded again (it=0, t=0), then k steps timed
+    launch set-up), the state uploaded again (it=0, t=0), then k steps timed
     with CUDA events on its stream.  Returns (seconds, state after k steps)."""
     from vac_gb300.engine import Engine
     e = Engine(params, snap.x, snap.w)

@@ -43,17 +43,21 @@ bool pair_applies(const FusedArgs& a, bool mhd) {
 }
 
 // Planes per CTA (z chunk) of a sweep over `tiles` column tiles and n planes
-// where the caller fixes none: grids of at least three waves (456 CTAs, three
-// per SM, each) in chunks of 32 or 16 planes take those; smaller ones the
-// longest chunk of at most 8 planes that still gives 350 CTAs, down to 2.
-// A CTA marches one plane in 3.7 us alone on its SM and in little more
-// beside two others, so a small grid is bound by the length of the march,
-// although every chunk predicts two planes beyond its own: a 64^3 sweep
-// takes 33 us in chunks of 3 (352 CTAs), 44 in chunks of 8 and 131 in
-// chunks of 32 (32 CTAs); 96^3 65 us with 8, 132 with 32; 127^3 114 with 8,
-// 126 with 16, 164 with 32.
+// where the caller fixes none: the longest of 24, 20, 16 and 12 planes that
+// gives at least three waves (456 CTAs, three per SM, each), else the longest
+// of at most 8 that gives 350 CTAs, down to 2.  Every chunk predicts two
+// planes beyond its own, but the march of one CTA is a serial chain (1.9 us a
+// plane alone on its SM, 2.8 beside two others), so a small grid wants many
+// short ones, and a large one enough of them that the last wave leaves few
+// slots idle.  Measured, us a sweep (periodic MHD): 64^3 26.9 with 4 planes,
+// 32.7 with 8 (131 with 32 at an earlier state of the kernel); 96^3 53 with 8,
+// 62 with 16; 128^3 96 with 8, 104 with 16, 119 with 32; 160^3 154 with 12,
+// 163 with 16; 192^3 240 with 20, 252 with 28, 283 with 64; 256^3 513 with
+// 24, 529 with 32, 563 with 64; 320^3 942 with 24, 992 with 64.  (A trial of
+// each chunk in a grid's first call, before, cost that call six steps and
+// found nothing better than this by more than 2 %.)
 static int pair_chunk(int tiles, int n) {
-  for (int z : {32, 16})
+  for (int z : {24, 20, 16, 12})
     if ((long long)tiles * ((n + z - 1) / z) >= 3 * 456) return z;
   for (int z : {8, 6, 4, 3})
     if ((long long)tiles * ((n + z - 1) / z) >= 350) return z;

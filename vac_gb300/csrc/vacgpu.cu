@@ -200,13 +200,7 @@ struct vacgpu_handle {
   bool fused;
   CUtensorMap tmap[2][2];  // [state buffer][x/z sweeps, y sweep]
   float* idxf[3];
-  int nzc;  // planes per CTA (0: the launcher's choice)
-  // z-chunk tuning of the fused 3-D sweep (results do not depend on the
-  // chunk): pending until the first vacgpu_step call, which times one step
-  // per candidate from a snapshot of the state and keeps the fastest
-  bool tuning;
-  int tncand;
-  int tcand[6];
+  int nzc;  // planes per CTA of the fused 3-D sweep (0: the launcher's choice)
   // asynchronous snapshots (vacgpu_snapshot_begin/wait): per slot the
   // mesh-ordered FP64 copy on the device, its page-locked host copy, and
   // the events that order the gather (on st) and the download (on cst)
@@ -726,55 +720,6 @@ void resume_dt(vacgpu_handle* h, int cur0, int steps) {
   run_dt_any(h);
 }
 
-// Issue k steps on the handle's stream without waiting: two-step units
-// are replayed from captured CUDA graphs keyed by (state buffer, parity of
-// it); h->cur follows the swaps of steps that execute.
-// z-chunk tuning of the fused 3-D sweep: one step per candidate from a
-// snapshot of the state (kept in the predictor buffer, which the fused
-// sweep does not use) and of the control block, restored after each trial,
-// so the run itself is untouched; the fastest candidate is kept.
-int tune_nzc(vacgpu_handle* h) {
-  h->tuning = false;
-  const size_t bytes = (size_t)h->g.vs * h->nw * h->elem;
-  const int cur0 = h->cur;
-  long long nl[VACGPU_K_NCLASS];
-  memcpy(nl, h->nlaunch, sizeof(nl));
-  Ctrl saved;
-  CK(cudaMemcpyAsync(&saved, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaMemcpyAsync(h->buf[2], h->buf[cur0], bytes, cudaMemcpyDeviceToDevice, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  cudaEvent_t e0, e1;
-  CK(cudaEventCreate(&e0));
-  CK(cudaEventCreate(&e1));
-  float best = 1e30f;
-  int nbest = h->nzc;
-  for (int i = 0; i < h->tncand; i++) {
-    h->nzc = h->tcand[i];
-    launch_call_ctl(h->ctrl, h->p, 1, 1e300, 0, h->st);
-    if (!dt_each_step(h)) run_dt<float>(h);
-    cudaEventRecord(e0, h->st);
-    run_step<float>(h, h->it_host & 1);
-    cudaEventRecord(e1, h->st);
-    CK(cudaEventSynchronize(e1));
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    if (ms < best) {
-      best = ms;
-      nbest = h->tcand[i];
-    }
-    CK(cudaMemcpyAsync(h->buf[cur0], h->buf[2], bytes, cudaMemcpyDeviceToDevice, h->st));
-    CK(cudaMemcpyAsync(h->ctrl, &saved, sizeof(Ctrl), cudaMemcpyHostToDevice, h->st));
-    CK(cudaStreamSynchronize(h->st));
-    h->cur = cur0;
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  memcpy(h->nlaunch, nl, sizeof(nl));
-  h->nzc = nbest;
-  CK(cudaGetLastError());
-  return 0;
-}
-
 // Captured graphs hold the launch arguments and hooks of their capture.
 void drop_graphs(vacgpu_handle* h) {
   for (int i = 0; i < 2; i++)
@@ -785,6 +730,9 @@ void drop_graphs(vacgpu_handle* h) {
       }
 }
 
+// Issue k steps on the handle's stream without waiting: two-step units
+// are replayed from captured CUDA graphs keyed by (state buffer, parity of
+// it); h->cur follows the swaps of steps that execute.
 int issue_steps(vacgpu_handle* h, int k, int it_base) {
   const int nsw = h->p.dimsplit ? h->p.ndim : 1;
   const bool graphs = !h->timing && h->st != nullptr &&
@@ -934,7 +882,6 @@ int vacgpu_internal_set_cur(vacgpu_handle* h, int cur) {
 // Server support: issue k steps that all execute (no stop condition in
 // between) without any host synchronisation.
 int vacgpu_internal_step_async(vacgpu_handle* h, int k) {
-  h->tuning = false;  // served solves keep the default z chunk
   if (h->fresh) {
     h->async_cur = h->cur;
     h->async_it = h->it_host;
@@ -1187,7 +1134,7 @@ int vacgpu_create(const vacgpu_params* p, vacgpu_handle** out) {
     vacgpu_destroy(h);
     return fail(std::string("device allocation failed: ") + cudaGetErrorString(e));
   }
-  h->nzc = 0;  // the launcher's choice, unless pinned or tuned
+  h->nzc = 0;  // the launcher's choice, unless pinned
   if (const char* nz = getenv("VACGPU_NZC")) h->nzc = atoi(nz) > 0 ? atoi(nz) : 32;
   h->fused = p->precision == VACGPU_PREC_MIXED && p->dimsplit &&
              (p->ndim == 2 || p->ndim == 3) && p->ndir == p->ndim &&
@@ -1204,12 +1151,6 @@ int vacgpu_create(const vacgpu_params* p, vacgpu_handle** out) {
         (ph.gmap[d][0] == GMAP_PERIODIC) != (ph.gmap[d][1] == GMAP_PERIODIC) ||
         ph.noflux[d][0] || ph.noflux[d][1])
       h->fused = false;
-  if (h->fused && p->ndim == 3 && !getenv("VACGPU_NZC") && g.ncell >= (1LL << 21)) {
-    static const int cands[6] = {8, 16, 24, 32, 48, 64};
-    for (int i = 0; i < 6; i++)
-      if (cands[i] < g.nx[2]) h->tcand[h->tncand++] = cands[i];
-    h->tuning = h->tncand > 1;
-  }
   if (h->fused) {
     bool ok = true;
     for (int i = 0; i < 2 && ok; i++)
@@ -1497,7 +1438,6 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
     return fail("the state is invalid after a timed-out device wait; upload a state first");
   if (h->any_special && !h->bound_fn) return fail(NO_SPECIAL);
   if (h->etaf && !h->eta_fn) return fail(NO_ETA);
-  if (h->tuning && maxsteps > 0 && !h->timing && tune_nzc(h)) return 1;
   const int nsw = h->p.dimsplit ? h->p.ndim : 1;
   const int start_cur = h->cur;
   begin_call(h, maxsteps, tstop);
@@ -1654,7 +1594,6 @@ int vacgpu_register_source_fn(vacgpu_handle* h, vacgpu_source_fn src,
   h->dtsp_fn = dt;
   h->src_user = user;
   h->ph.src_hook = src != nullptr;
-  if (src) h->tuning = false;  // the split kernels run; no z chunk to tune
   if (src || dt) {
     // the hooks replace a built-in source
     h->ph.src_id = VACGPU_SRC_NONE;
