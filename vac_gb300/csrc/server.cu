@@ -84,7 +84,7 @@ namespace {
 
 void finish(vacgpu_server* s, Req* r, bool ok, const std::string& err) {
   if (ok) {
-    r->result.resize(r->w.size());
+    r->result.swap(r->w);  // the state's own pages: the upload is long done
     double dt;
     int fin;
     if (vacgpu_step(r->h, 0, 1e300, &r->t_sim, &r->it, &dt, &fin) ||
