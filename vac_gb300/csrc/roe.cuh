@@ -52,6 +52,7 @@ struct RoeSweep {
     // 1/SIGN(sr,B_idim), v^2 and v^2/2+(2-gamma)/(gamma-1)*cs2, formed once
     // per face instead of in each of rtimes' products
     R sgn, csr, isrs, vv, v2a2;
+    typename PH::Den srd;  // FP64: quotients by sr
   };
 
   // Fortran SIGN(a,b), MAX and MIN as the oracle's selects
@@ -88,7 +89,8 @@ struct RoeSweep {
   template <int il>
   static __device__ __forceinline__ void wave(const SweepArgs& a, const R* wL,
                                               const R* wR, int d, double smallp,
-                                              D qdt, R dxs, const R* bd,
+                                              D qdt, R dxs,
+                                              const typename PH::Den& dxd, const R* bd,
                                               Face& f, D* am) {
     const R rL = wL[0], rR = wR[0];
     const R v = f.v[d];
@@ -235,7 +237,7 @@ struct RoeSweep {
     if constexpr (sizeof(R) == 4)
       adt = aa * (R(qdt) * R(2) / dxs);
     else
-      adt = aa * R(qdt) * R(2) / dxs;
+      adt = PH::div(aa * R(qdt) * R(2), dxd);
     if (te == VACGPU_ENTROPY_HARTEN || te == VACGPU_ENTROPY_POWELL)
       smalla = smalla * R(qdt) * R(2) / dxs;
     if (il < 2) am[il] = fabs(adt);
@@ -488,14 +490,15 @@ struct RoeSweep {
       f.cs = D(c);
       f.rhodv = D(((double)wR[1 + d] / dR - (double)wL[1 + d] / dL) / c);
     }
-    wave<0>(a, wL, wR, d, smallp, qdt, dxs, bd, f, am);
-    wave<1>(a, wL, wR, d, smallp, qdt, dxs, bd, f, am);
-    wave<2>(a, wL, wR, d, smallp, qdt, dxs, bd, f, am);
-    if (NW > 3) wave<(NW > 3 ? 3 : 0)>(a, wL, wR, d, smallp, qdt, dxs, bd, f, am);
-    if (NW > 4) wave<(NW > 4 ? 4 : 0)>(a, wL, wR, d, smallp, qdt, dxs, bd, f, am);
-    if (NW > 5) wave<(NW > 5 ? 5 : 0)>(a, wL, wR, d, smallp, qdt, dxs, bd, f, am);
-    if (NW > 6) wave<(NW > 6 ? 6 : 0)>(a, wL, wR, d, smallp, qdt, dxs, bd, f, am);
-    if (NW > 7) wave<(NW > 7 ? 7 : 0)>(a, wL, wR, d, smallp, qdt, dxs, bd, f, am);
+    const typename PH::Den dxd = PH::den(dxs);
+    wave<0>(a, wL, wR, d, smallp, qdt, dxs, dxd, bd, f, am);
+    wave<1>(a, wL, wR, d, smallp, qdt, dxs, dxd, bd, f, am);
+    wave<2>(a, wL, wR, d, smallp, qdt, dxs, dxd, bd, f, am);
+    if (NW > 3) wave<(NW > 3 ? 3 : 0)>(a, wL, wR, d, smallp, qdt, dxs, dxd, bd, f, am);
+    if (NW > 4) wave<(NW > 4 ? 4 : 0)>(a, wL, wR, d, smallp, qdt, dxs, dxd, bd, f, am);
+    if (NW > 5) wave<(NW > 5 ? 5 : 0)>(a, wL, wR, d, smallp, qdt, dxs, dxd, bd, f, am);
+    if (NW > 6) wave<(NW > 6 ? 6 : 0)>(a, wL, wR, d, smallp, qdt, dxs, dxd, bd, f, am);
+    if (NW > 7) wave<(NW > 7 ? 7 : 0)>(a, wL, wR, d, smallp, qdt, dxs, dxd, bd, f, am);
   }
 
   // R(iw,il)*q at the Roe state (rtimes, src/vacphys.mhdroe.t:284-449 and
@@ -606,16 +609,17 @@ struct RoeSweep {
       switch (il) {
         case 0:
         case 1:
-          return +q * f.as * sqrt(f.cs2) * bw / f.sr;
+          return PH::div(+q * f.as * sqrt(f.cs2) * bw, f.srd);
         case 2:
         case 3:
-          return -q * f.af * sqrt(f.cs2) * bw / f.sr;
+          return PH::div(-q * f.af * sqrt(f.cs2) * bw, f.srd);
         case 4:
         case 5:
           return R(0);
         default:
-          if (c == I) return -q * f.b[J] / R(fsign(f.sr, f.b[d]));
-          return +q * f.b[I] / R(fsign(f.sr, f.b[d]));
+          // (divided by SIGN(sr,b_idim): the sign moves to the numerator)
+          if (c == I) return PH::div(-q * f.b[J] * R(fsign(1.0, f.b[d])), f.srd);
+          return PH::div(+q * f.b[I] * R(fsign(1.0, f.b[d])), f.srd);
       }
     } else {
       const bool shear = il >= 3;
@@ -665,6 +669,7 @@ struct RoeSweep {
     for (int iw = 0; iw < NW; iw++) F[iw] = R(0.5) * (fL[iw] + fR[iw]);
     const R dxs = PH::dx(a.a, d, cl[d]) + PH::dx(a.a, d, cl[d] + 1);
     decompose(a, wL, wR, d, qsmallp, qdt, dxs, f, am);
+    if (MHD && sizeof(R) == 8) f.srd = PH::den(f.sr);
   }
 
   // dvolume(ix) = dx_1*dx_2*dx_3 (gridsetup1, src/vacgrid.t:573-576)
@@ -922,6 +927,9 @@ struct RoeSweep {
       S::to_cons(a, acc);
     }
     const R dv0 = dvol(a, c);
+    // (FP64: the NW^2 quotients by dv0 share its reciprocal; with those by
+    // dx(i)+dx(j) and sr a 160x144 step takes 155 us, 171 before)
+    const typename PH::Den dvd = PH::den(dv0);
     for (int d = a.d0; d <= a.d1; d++) {
       const R* buf = (const R*)a.faces + (long long)(d - a.d0) * a.face_stride;
       const long long nf = face_count(a.g, d);
@@ -945,7 +953,7 @@ struct RoeSweep {
 #pragma unroll
           for (int iw = 0; iw < NW; iw++) {
             const R* r = buf + (long long)(NW + il * NW + iw) * nf;
-            acc[iw] = acc[iw] + (r[fp] - r[fm]) / dv0;
+            acc[iw] = acc[iw] + PH::div(r[fp] - r[fm], dvd);
           }
       }
     }
