@@ -928,7 +928,7 @@ struct RoeSweep {
     }
     const R dv0 = dvol(a, c);
     // (FP64: the NW^2 quotients by dv0 share its reciprocal; with those by
-    // dx(i)+dx(j) and sr a 160x144 step takes 155 us, 171 before)
+    // dx(i)+dx(j) and sr a job of 40 steps on 160x144 takes 6.5 ms, 7.1 before)
     const typename PH::Den dvd = PH::den(dv0);
     for (int d = a.d0; d <= a.d1; d++) {
       const R* buf = (const R*)a.faces + (long long)(d - a.d0) * a.face_stride;
