@@ -323,3 +323,33 @@ def test_fused_roe_against_oracle_and_split(gpu_lib, monkeypatch, name, nx, lim,
     e = Engine(pm, s.x, s.w)
     e.step(2)
     assert e.kernel_stats()["sweep"][0] == 0
+
+
+def _hd3(nx, seed=8):
+    """Gas with the random modes' density and velocity on a box of cubic cells."""
+    s = inistate.random_modes(max(nx), seed=seed, p0=0.5)
+    w = s.w[(slice(0, 4),) + tuple(slice(0, n) for n in nx)]
+    x = inistate.domain_grid(nx, (0.0,) * 3, tuple(n / max(nx) for n in nx))
+    w = inistate.conserve_hd(w[0], [w[1 + d] / w[0] for d in range(3)],
+                             np.full(nx, 0.5), 1.4)
+    return inistate._snap(x, w, 1.4, False, 3, "random-mode gas")
+
+
+HD3_CASES = [
+    ("hd3-33x18x9-cont", (33, 18, 9), "woodward", "cont"),
+    ("hd3-45x9x17-reflect", (45, 9, 17), "minmod", "symm"),
+    ("hd3-31x12x10-cont", (31, 12, 10), "minmod", "cont"),
+    ("hd3-32x12x10-reflect", (32, 12, 10), "woodward", "symm"),
+    ("hd3-32x24x30-cont", (32, 24, 30), "woodward", "cont"),
+    ("hd3-65x20x11-periodic", (65, 20, 11), "woodward", "periodic"),
+    ("hd3-64x33x36-periodic", (64, 33, 36), "minmod", "periodic"),
+]
+
+
+@pytest.mark.parametrize("name,nx,lim,bc", HD3_CASES, ids=[c[0] for c in HD3_CASES])
+def test_fused_gas_3d(gpu_lib, monkeypatch, name, nx, lim, bc):
+    """3-D gas on the pair sweep, whose cells carry five variables where MHD's
+    carry eight: odd and even widths, each kind of face."""
+    test_fused_against_oracle_and_split(
+        gpu_lib, monkeypatch, name, lambda: _hd3(nx), lim, bc, 8,
+        (lambda p: reflecting(p, 3)) if bc == "symm" else None)

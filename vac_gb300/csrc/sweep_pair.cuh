@@ -714,19 +714,23 @@ struct PairSweep {
         if (fix_m && j == 0) {
 #pragma unroll
           for (int v = 0; v < NW; v++) w1p[v] = wflip(w1[v], v, a.asymm_lo[AM]);
-          bzm1 = w1p[5 + AM];
+          if constexpr (MHD) bzm1 = w1p[5 + AM];
         }
         if (fix_m && j == nM) {
 #pragma unroll
           for (int v = 0; v < NW; v++) w1[v] = wflip(w1p[v], v, a.asymm_hi[AM]);
         }
-        // an odd mesh width: the first ghost column is the second cell of the
-        // last pair, whose B_x the first cell's div B takes from registers
-        if (fix_x && ix0 + 1 == nX) {
-          const float lo = f2lo(w1[5]);
-          w1[5] = f2m(lo, f2lo(wflip(w1[5], 5, a.asymm_hi[0])));
+        // (gas has five variables: indices from 5 on are MHD's alone)
+        if constexpr (MHD) {
+          // an odd mesh width: the first ghost column is the second cell of
+          // the last pair, whose B_x the first cell's div B takes from
+          // registers
+          if (fix_x && ix0 + 1 == nX) {
+            const float lo = f2lo(w1[5]);
+            w1[5] = f2m(lo, f2lo(wflip(w1[5], 5, a.asymm_hi[0])));
+          }
+          bz = w1[5 + AM];
         }
-        bz = w1[5 + AM];
         if (ring) {
           if (!(xhi && lx0 >= xe)) st2(wb(sm, j, 0, ly, lx0), w1[5]);
           if (xlo && lx0 == 0)
@@ -866,7 +870,7 @@ struct PairSweep {
               }
             }
           }
-          bz = w1[5 + AM];
+          if constexpr (MHD) bz = w1[5 + AM];
 #pragma unroll
           for (int v = 0; v < NW; v++) hl_[v] = hlv[v];
           if (ring) {
