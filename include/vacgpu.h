@@ -328,7 +328,10 @@ int vacgpu_register_source(vacgpu_handle* h, int source_id,
  * read: *qdt = qdt*(idimmax-idimmin+1)/ndim of the call (src/vactvdlf.t:85,
  * 292), *box.qt = qt = t.  The hook enqueues device work on `stream` that
  * updates w on the cells of box (the arrays use box's indexing), must not
- * synchronise, and returns 0 (non-zero fails the call that issued it). */
+ * synchronise, and returns 0 (non-zero fails the call that issued it).  The
+ * engine issues steps ahead of the device, so hooks are also called for steps
+ * behind a stop, which do nothing: whatever the hook's kernels then write to
+ * w is dropped. */
 typedef struct vacgpu_source_args {
   vacgpu_region box;       /* the mesh; box.qt: device pointer to qt        */
   const double* qdt;       /* device: the source's time step                */

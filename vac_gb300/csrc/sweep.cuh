@@ -610,10 +610,11 @@ struct Sweep {
 
   // addsource (src/vac.t:575-605 after specialsource) as a pass of its own
   // when the user's specialsource hook runs between the flux update and
-  // it: w += addsource(wCT) on the mesh, with the operations the predictor
-  // (pred) or corrector kernel performs in place otherwise.
+  // it: wout = w + addsource(wCT) on the mesh (wout may be w), with the
+  // operations the predictor (pred) or corrector kernel performs in place
+  // otherwise.
   static __device__ void source_pass(const SweepArgs& a, const T* __restrict__ wct,
-                                     T* __restrict__ w, int pred) {
+                                     const T* w, T* wout, int pred) {
     const Ctrl* ctrl = a.ctrl;
     if (ctrl->done) return;
     long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -631,7 +632,7 @@ struct Sweep {
     }
     add_sources(a, src_qdt(a, pred != 0), wc, wct + off, st, c, acc);
 #pragma unroll
-    for (int iw = 0; iw < NW; iw++) w[off + iw * vs] = T(acc[iw]);
+    for (int iw = 0; iw < NW; iw++) wout[off + iw * vs] = T(acc[iw]);
   }
 
   // getpthermal's one-time smallp: min/max of the unclipped pressure on the
@@ -1064,8 +1065,8 @@ void launch_face_dir(const SweepArgs& a, const typename PH::T* w1,
 template <class PH, int NDIM, int NDIR, bool MHD>
 __global__ void __launch_bounds__(128)
     k_source_pass(SweepArgs a, const typename PH::T* __restrict__ wct,
-                  typename PH::T* __restrict__ w, int pred) {
-  Sweep<PH, NDIM, NDIR, MHD>::source_pass(a, wct, w, pred);
+                  const typename PH::T* w, typename PH::T* wout, int pred) {
+  Sweep<PH, NDIM, NDIR, MHD>::source_pass(a, wct, w, wout, pred);
 }
 
 template <class PH, int NDIM, int NDIR, bool MHD>
@@ -1171,10 +1172,10 @@ struct Launch {
     VACGPU_DISPATCH(a, KC);
 #undef KC
   }
-  static void source_pass(const SweepArgs& a, const T* wct, T* w, int pred,
+  static void source_pass(const SweepArgs& a, const T* wct, const T* w, T* wout, int pred,
                           cudaStream_t st) {
     const unsigned nb = grid_for(a.g.ncell, 128);
-#define KC(D, C, M) k_source_pass<PH, D, C, M><<<nb, 128, 0, st>>>(a, wct, w, pred)
+#define KC(D, C, M) k_source_pass<PH, D, C, M><<<nb, 128, 0, st>>>(a, wct, w, wout, pred)
     VACGPU_DISPATCH(a, KC);
 #undef KC
   }
@@ -1304,8 +1305,9 @@ struct Launch {
     Launch<PH>::ghost(s, w, st, true);                                       \
   }                                                                          \
   void launch_source_pass_##SUF(const SweepArgs& s, const PH::T* wct,        \
-                                PH::T* w, int pred, cudaStream_t st) {       \
-    Launch<PH>::source_pass(s, wct, w, pred, st);                            \
+                                const PH::T* w, PH::T* wout, int pred,       \
+                                cudaStream_t st) {                           \
+    Launch<PH>::source_pass(s, wct, w, wout, pred, st);                      \
   }                                                                          \
   void launch_pminmax_##SUF(const SweepArgs& s, const PH::T* w,              \
                             cudaStream_t st) {                               \

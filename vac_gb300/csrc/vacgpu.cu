@@ -148,6 +148,7 @@ struct vacgpu_handle {
   vacgpu_source_fn src_fn;       // the user's specialsource
   vacgpu_dtspecial_fn dtsp_fn;   // the user's getdt_special
   void* src_user;
+  void* srcbuf;      // the corrector's output that the user's source updates
   double* etaf;      // its eta field, gradeta (compactres) and the current
   double* gradetaf[3];
   double* curf[3];
@@ -448,9 +449,13 @@ static void mesh_region(const vacgpu_handle* h, vacgpu_region& r) {
 // then addsource as a pass of its own (the predictor and corrector kernels
 // leave it out while a hook is installed).  pred: after the Hancock
 // predictor (qdt = dt/2); half: qtC = t+dt/2 (the corrector of twostep).
+// The hook updates w, and the pass stores to wout.  The user's kernels also
+// run for steps that were issued but do nothing (behind a stop), where the
+// engine's own kernels return: such a step's wout may be the state, so the
+// corrector's w is a buffer of its own (src_target).
 template <typename T>
 void source_hook(vacgpu_handle* h, const SweepArgs& a, int pred, int half, const T* wct,
-                 T* w) {
+                 T* w, T* wout) {
   if (!h->src_fn || !h->p.sourceunsplit) return;
   kbegin(h, VACGPU_K_CONTROL);
   launch_src_args(h->ctrl, pred, half, a.d1 - a.d0 + 1, h->p.ndim, h->st);
@@ -467,14 +472,20 @@ void source_hook(vacgpu_handle* h, const SweepArgs& a, int pred, int half, const
   if (h->src_fn(h->src_user, &s, (void*)h->st)) h->hook_failed = true;
   kbegin(h, pred ? VACGPU_K_PREDICT : VACGPU_K_CORRECT);
   if (sizeof(T) == 8)
-    launch_source_pass_fp64(a, (const double*)wct, (double*)w, pred, h->st);
+    launch_source_pass_fp64(a, (const double*)wct, (const double*)w, (double*)wout, pred, h->st);
   else if (h->pmode == 1)
-    launch_source_pass_mixedf64(a, (const float*)wct, (float*)w, pred, h->st);
+    launch_source_pass_mixedf64(a, (const float*)wct, (const float*)w, (float*)wout, pred, h->st);
   else if (h->pmode == 2)
-    launch_source_pass_mixedf32(a, (const float*)wct, (float*)w, pred, h->st);
+    launch_source_pass_mixedf32(a, (const float*)wct, (const float*)w, (float*)wout, pred, h->st);
   else
-    launch_source_pass_mixed(a, (const float*)wct, (float*)w, pred, h->st);
+    launch_source_pass_mixed(a, (const float*)wct, (const float*)w, (float*)wout, pred, h->st);
   kend(h);
+}
+
+// what the corrector writes: the user's source follows in the same buffer
+template <typename T>
+T* src_target(vacgpu_handle* h, T* wout) {
+  return h->src_fn && h->p.sourceunsplit ? (T*)h->srcbuf : wout;
 }
 
 // getboundary of a pass's output where the pass has not filled its ghost
@@ -531,6 +542,7 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
     kend(h);
     wc = base = (const T*)h->wold;
   }
+  T* wcor = src_target(h, wout);
   const bool roe = h->p.typefull == VACGPU_TVDMU || h->p.typefull == VACGPU_TVDMU1;
   if (h->p.typefull == VACGPU_TVDLF1 || h->p.typefull == VACGPU_TVDMU1) {
     // typepred1='nul': onestep, the corrector alone with wCT = w
@@ -539,36 +551,36 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
     kbegin(h, VACGPU_K_CORRECT);
     if (sizeof(T) == 8 && roe)
       launch_correct_roe_fp64(a, (const double*)w, (const double*)w,
-                              (const double*)w, (double*)wout, h->st);
+                              (const double*)w, (double*)wcor, h->st);
     else if (sizeof(T) == 8)
       launch_correct_fp64(a, (const double*)w, (const double*)w,
-                          (const double*)w, (double*)wout, h->st);
+                          (const double*)w, (double*)wcor, h->st);
     else if (roe)
       launch_correct_roe_mixed(a, (const float*)w, (const float*)w,
-                               (const float*)w, (float*)wout, h->st);
+                               (const float*)w, (float*)wcor, h->st);
     else
       launch_correct_mixed(a, (const float*)w, (const float*)w,
-                           (const float*)w, (float*)wout, h->st);
+                           (const float*)w, (float*)wcor, h->st);
     kend(h);
-    source_hook<T>(h, a, 0, 0, w, wout);
+    source_hook<T>(h, a, 0, 0, w, wcor, wout);
     after_pass(h, a, wout, 2);
   } else if (sizeof(T) == 8) {
     if (h->p.sourceunsplit) eta_hook(h, a, w, 0);
     kbegin(h, VACGPU_K_PREDICT);
     launch_predict_fp64(a, (const double*)w, (double*)w1, h->st);
     kend(h);
-    source_hook<T>(h, a, 1, 0, w, w1);
+    source_hook<T>(h, a, 1, 0, w, w1, w1);
     after_pass(h, a, w1, 1);
     if (h->p.sourceunsplit) eta_hook(h, a, w1, 0);
     kbegin(h, VACGPU_K_CORRECT);
     if (roe)
       launch_correct_roe_fp64(a, (const double*)wc, (const double*)w1,
-                              (const double*)base, (double*)wout, h->st);
+                              (const double*)base, (double*)wcor, h->st);
     else
       launch_correct_fp64(a, (const double*)wc, (const double*)w1,
-                          (const double*)base, (double*)wout, h->st);
+                          (const double*)base, (double*)wcor, h->st);
     kend(h);
-    source_hook<T>(h, a, 0, 1, (const T*)w1, wout);
+    source_hook<T>(h, a, 0, 1, (const T*)w1, wcor, wout);
     after_pass(h, a, wout, 2);
   } else if (h->fused && h->pmode == 0 && d0 == d1 && !h->src_fn) {
     kbegin(h, VACGPU_K_SWEEP);
@@ -581,22 +593,23 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
     const float* fwc = (const float*)wc;
     float* fw1 = (float*)w1;
     float* fo = (float*)wout;
+    float* fc = (float*)wcor;
     const float* fb = (const float*)base;
 #define MIXED_SWEEP(SUF)                                \
   if (h->p.sourceunsplit) eta_hook(h, a, fw, 0);        \
   kbegin(h, VACGPU_K_PREDICT);                          \
   launch_predict_##SUF(a, fw, fw1, h->st);              \
   kend(h);                                              \
-  source_hook<T>(h, a, 1, 0, w, w1);                    \
+  source_hook<T>(h, a, 1, 0, w, w1, w1);                \
   after_pass(h, a, fw1, 1);                             \
   if (h->p.sourceunsplit) eta_hook(h, a, fw1, 0);       \
   kbegin(h, VACGPU_K_CORRECT);                          \
   if (roe)                                              \
-    launch_correct_roe_mixed(a, fwc, fw1, fb, fo, h->st); \
+    launch_correct_roe_mixed(a, fwc, fw1, fb, fc, h->st); \
   else                                                  \
-    launch_correct_##SUF(a, fwc, fw1, fb, fo, h->st);   \
+    launch_correct_##SUF(a, fwc, fw1, fb, fc, h->st);   \
   kend(h);                                              \
-  source_hook<T>(h, a, 0, 1, (const T*)w1, wout);       \
+  source_hook<T>(h, a, 0, 1, (const T*)w1, wcor, wout); \
   after_pass(h, a, fo, 2);
     switch (h->pmode) {
       case 1: MIXED_SWEEP(mixedf64) break;
@@ -1597,6 +1610,14 @@ int vacgpu_register_source_fn(vacgpu_handle* h, vacgpu_source_fn src,
   if (h->st) CK(cudaStreamSynchronize(h->st));
   drop_graphs(h);
   if (src && !h->faces && alloc_faces(h)) return 1;
+  if (src && h->p.sourceunsplit && !h->srcbuf) {
+    const size_t bytes = h->elem * (size_t)h->g.vs * h->nw;
+    if (cudaMalloc(&h->srcbuf, bytes) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return fail("device allocation of the source hook's buffer failed");
+    }
+    CK(cudaMemsetAsync(h->srcbuf, 0, bytes, h->st));
+  }
   h->src_fn = src;
   h->dtsp_fn = dt;
   h->src_user = user;
@@ -1629,6 +1650,7 @@ void vacgpu_destroy(vacgpu_handle* h) {
   cudaFree(h->wold);
   cudaFree(h->fixb);
   cudaFree(h->faces);
+  cudaFree(h->srcbuf);
   cudaFree(h->etaf);
   for (int k = 0; k < 3; k++) {
     cudaFree(h->curf[k]);

@@ -265,8 +265,9 @@ struct SweepArgs {
                             const T* base, T* wout, cudaStream_t st);        \
   void launch_ghost_##SUF(const SweepArgs& s, T* w, cudaStream_t st);        \
   void launch_ghost_yz_##SUF(const SweepArgs& s, T* w, cudaStream_t st);     \
-  void launch_source_pass_##SUF(const SweepArgs& s, const T* wct, T* w,     \
-                                int pred, cudaStream_t st);                  \
+  void launch_source_pass_##SUF(const SweepArgs& s, const T* wct,            \
+                                const T* w, T* wout, int pred,               \
+                                cudaStream_t st);                            \
   void launch_pminmax_##SUF(const SweepArgs& s, const T* w, cudaStream_t st); \
   void launch_cell_cmax_##SUF(const SweepArgs& s, const T* w,                \
                               cudaStream_t st);                              \
