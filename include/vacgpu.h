@@ -276,7 +276,8 @@ typedef struct vacgpu_region {
  * before the next region (getboundary's order).  It enqueues device work
  * on `stream` (a cudaStream_t) that writes the region's cells of the
  * variables in iw_mask, must not synchronise, and returns 0 (non-zero
- * fails the call that issued the fill). */
+ * fails the call that issued the fill).  It may also run again on a filled
+ * state with the same qt (steps issued behind a stop, which do nothing). */
 typedef int (*vacgpu_bound_fn)(void* user, void* w, const vacgpu_region* r,
                                void* stream);
 

@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from oracle.oracle import Oracle
+from tests import test_special_bound as tb
 from tests import test_special_source as ts
 from vac_gb300 import inistate
 from vac_gb300.engine import Engine
@@ -72,6 +73,40 @@ def test_source_hook_where_every_step_needs_the_passes(gpu_lib):
     p = inistate.params_for(s)
     e = Engine(p, s.x, s.w, source=(ds, None, None))
     o = Oracle(p, s.x, s.w, source=(hs, None, ts._e_index(p)))
+    e.step(12)
+    o.step(12)
+    assert (e.it, e.t) == (12, o.t) and same(e.state(), o.state())
+
+
+def test_special_faces_keep_their_time_at_a_stop(gpu_lib):
+    """The ghost values of a time-dependent 'special' face after a stop are
+    those of the stop's time, also where steps issued behind it filled the
+    face again."""
+    Lh, hfn = tb._host_hook()
+    Ld, dfn = tb._device_hook()
+    s = inistate.riemann_2d(32, 3)
+    p = inistate.params_for(s, bc="cont")
+    tb._special([0])(p)
+    # (a step after an even it starts with the x sweep, which reads the face)
+    e = Engine(p, s.x, s.w, bound=(dfn, None))
+    e.step(6)
+    tstop = 0.999 * e.t
+    e = Engine(p, s.x, s.w, bound=(dfn, None))
+    o = Oracle(p, s.x, s.w, bound=(hfn, None))
+    assert not e.step(13, tstop=tstop) and e.it == 6
+    e.step(4)
+    o.step(10)
+    assert (e.it, e.t) == (10, o.t) and same(e.state(), o.state())
+
+
+def test_special_faces_where_every_step_needs_the_passes(gpu_lib):
+    Lh, hfn = tb._host_hook()
+    Ld, dfn = tb._device_hook()
+    s = dust()
+    p = inistate.params_for(s, bc="cont")
+    tb._special([0], ivars=[0])(p)
+    e = Engine(p, s.x, s.w, bound=(dfn, None))
+    o = Oracle(p, s.x, s.w, bound=(hfn, None))
     e.step(12)
     o.step(12)
     assert (e.it, e.t) == (12, o.t) and same(e.state(), o.state())

@@ -9,8 +9,11 @@ namespace vacgpu {
 
 __global__ void k_dt_begin(Ctrl* c, int ndim) { dt_begin_dev(c, ndim); }
 // getboundary's qt: t (before the loop), qt+qdt = t+dt/2 after the
-// predictor and t+dt after the corrector (src/vac.t:54,567)
+// predictor and t+dt after the corrector (src/vac.t:54,567).  A step that
+// does nothing (done) keeps the last fill's: the user's kernels run in it all
+// the same, and fill the state's faces again.
 __global__ void k_set_qt(Ctrl* c, int mode) {
+  if (c->done) return;
   c->qt = mode == 0 ? c->t : mode == 1 ? c->t + c->dt / 2 : c->t + c->dt;
 }
 __global__ void k_smallp(Ctrl* c, int mhd, double coeff) {
