@@ -110,3 +110,19 @@ def test_special_faces_where_every_step_needs_the_passes(gpu_lib):
     e.step(12)
     o.step(12)
     assert (e.it, e.t) == (12, o.t) and same(e.state(), o.state())
+
+
+def test_removed_dt_hook_limits_nothing(gpu_lib):
+    """Without the getdt_special hook its last limit no longer counts."""
+    from vac_gb300.engine import _ck, lib
+    Lh, hs, hd = ts._host_hook()
+    Ld, ds, dd = ts._device_hook()
+    s = inistate.orszag_tang(24)
+    p = inistate.params_for(s)
+    e = Engine(p, s.x, s.w, source=(None, dd, None))
+    e.step(3)
+    w = e.state()
+    _ck(lib().vacgpu_register_source_fn(e.h, None, None, None), "vacgpu_register_source_fn")
+    e.step(1)
+    limited = 0.05 / (0.001 + np.abs(w[1] / w[0]).max())
+    assert e.dt > 1.2 * limited

@@ -1619,6 +1619,11 @@ int vacgpu_register_source_fn(vacgpu_handle* h, vacgpu_source_fn src,
     CK(cudaMemsetAsync(h->srcbuf, 0, bytes, h->st));
   }
   h->src_fn = src;
+  if (!dt && h->dtsp_fn) {
+    // without the hook its last limit counts no more
+    double v = BIGD;
+    CK(cudaMemcpy(&h->ctrl->dtspecial, &v, sizeof(double), cudaMemcpyHostToDevice));
+  }
   h->dtsp_fn = dt;
   h->src_user = user;
   h->ph.src_hook = src != nullptr;
