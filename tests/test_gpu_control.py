@@ -86,3 +86,69 @@ def test_call_lengths_and_stops(gpu_lib, name, mk, lim, bc, prec):
     e = Engine(p, s.x, s.w)
     assert e.step(400) and e.it == mid
     assert e.step(5) and e.it == mid
+
+
+# cells of the speed checks and their steps: a launch-bound grid
+N_DUST, STEPS_DUST = 64, 400
+
+
+def dust_and_gas():
+    """Pressureless gas that flows along x (no wave speed along y, so each
+    step's dt needs the cell-centred pass) and ordinary gas on one grid."""
+    from tests.test_gpu_skipped_steps import dust
+    return dust(N_DUST, N_DUST), inistate.riemann_2d(N_DUST, 3)
+
+
+@pytest.mark.parametrize("prec", [abi.PREC_FP64, abi.PREC_MIXED])
+def test_passes_at_every_step_cost_their_launches(gpu_lib, prec):
+    """Steps that need the cell-centred passes cost six launches more than
+    others, not a round trip to the host each: no more than 40 us a step, and
+    a served run no more than a run alone, its set-up and one more chunk."""
+    import time
+    sd, sg = dust_and_gas()
+    best, eng = {}, {}
+    for name, s in (("dust", sd), ("gas", sg)):
+        e = eng[name] = Engine(inistate.params_for(s, precision=prec), s.x, s.w)
+        for _ in range(4):
+            e.upload(s.w)
+            t0 = time.perf_counter()
+            e.step(STEPS_DUST)
+            best[name] = min(best.get(name, 1e9), time.perf_counter() - t0)
+            assert e.it == STEPS_DUST
+    assert best["dust"] - best["gas"] <= 40e-6 * STEPS_DUST, best
+    p = inistate.params_for(sd, precision=prec)
+    srv = Server(hbm_budget_bytes=1e9, max_active=2, steps_per_chunk=16)
+    t0 = time.perf_counter()
+    st, t, it, tts = srv.result(srv.submit(p, sd.x, sd.w, STEPS_DUST), wait=120.0)
+    served = time.perf_counter() - t0
+    srv.close()
+    assert it == STEPS_DUST and t == eng["dust"].t and same(st, eng["dust"].state())
+    assert served <= 2 * best["dust"] + 0.05, (served, best)
+    if prec == abi.PREC_FP64:
+        o = Oracle(p, sd.x, sd.w)
+        o.step(STEPS_DUST)
+        assert t == o.t and same(st, o.state())
+
+
+@pytest.mark.parametrize("chunk", [1, 7, 16])
+def test_served_gas_that_stalls_late(gpu_lib, chunk):
+    """Wave speeds along y that die out (the gas that moved along y leaves
+    through an outflow face; below 1e-99 a speed sets no dt): the passes are
+    needed from the middle of the run on."""
+    from tests.test_gpu_skipped_steps import dust
+    s = dust(12, 9)
+    s.w[2, -1, :] = 1e-80 * s.w[0, -1, :]
+    p = inistate.params_for(s, bc="cont")
+    o = Oracle(p, s.x, s.w)
+    o.step(20)
+    assert np.abs(o.state()[2]).max() > 1e-97
+    o.step(40)
+    assert np.abs(o.state()[2]).max() < 1e-101
+    srv = Server(hbm_budget_bytes=1e9, max_active=2, steps_per_chunk=chunk)
+    st, t, it, _ = srv.result(srv.submit(p, s.x, s.w, 60), wait=60.0)
+    srv.close()
+    assert (it, t) == (60, o.t) and same(st, o.state())
+    e = Engine(p, s.x, s.w)
+    for n in (1, 2, 30, 27):
+        e.step(n)
+    assert (e.it, e.t) == (60, o.t) and same(e.state(), o.state())

@@ -266,7 +266,7 @@ __device__ __forceinline__ void step_end_dev(Ctrl* c, int ndim, int toggle) {
 // (dt_begin, then dt_end).  A step that does need the cell-centred passes
 // (its dtcourant is unset: a first step, or wave speeds that gave none) is
 // left to the host: done = 4 stops the kernels issued after it until the
-// host has run those passes (resume_dt in vacgpu.cu).
+// host goes on with those passes in every step (dt_passes in vacgpu.cu).
 __device__ __forceinline__ void choose_dt_dev(CtrlHead* c, Ctrl* k, int ndim,
                                               const DtEndArgs& p) {
   __shared__ int need;

@@ -28,7 +28,7 @@
 
 int vacgpu_internal_fail(const char* msg);
 int vacgpu_internal_step_async(vacgpu_handle* h, int k);
-int vacgpu_internal_steps_left(vacgpu_handle* h, int* left);
+int vacgpu_internal_steps_left(vacgpu_handle* h, int* left, int* passes);
 void* vacgpu_internal_stream(vacgpu_handle* h);
 size_t vacgpu_internal_device_bytes(const vacgpu_params* p);
 
@@ -50,6 +50,7 @@ struct Req {
   vacgpu_handle* h = nullptr;
   cudaEvent_t ev = nullptr;
   int issued = 0;
+  bool look = true;  // read back how far the next finished chunk got
   int state = 0;  // 0 queued, 1 active, 2 done, 3 failed
   std::vector<double> result;
   double t_done = 0.0, t_sim = 0.0;
@@ -175,10 +176,15 @@ void worker_loop(vacgpu_server* s) {
       }
       progressed = true;
       bool ok = true;
-      if (r->issued == r->nsteps) {
-        int left = 0;  // steps that wait for the first-step passes
-        ok = vacgpu_internal_steps_left(r->h, &left) == 0;
+      // Steps may wait for the first-step passes: after a run's first chunk
+      // (gas with no wave speed along one axis waits at its second step) and
+      // at its end, so that a run is issued twice at most; where every step
+      // has the passes, after each chunk.
+      if (r->issued && (r->look || r->issued == r->nsteps)) {
+        int left = 0, passes = 0;
+        ok = vacgpu_internal_steps_left(r->h, &left, &passes) == 0;
         r->issued -= left;
+        r->look = passes;
       }
       if (!ok || r->issued < r->nsteps) {
         const int k = r->nsteps - r->issued < s->chunk ? r->nsteps - r->issued : s->chunk;

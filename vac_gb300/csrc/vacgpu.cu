@@ -158,8 +158,11 @@ struct vacgpu_handle {
   unsigned special[VACGPU_MAXB];  // per region: bit iw 'special'
   double* xg[3];     // cell centres over the ghost box (specialbound hooks)
   int cur;           // which of buf[0], buf[1] holds the state
-  bool fresh;        // no step has run since the upload
-  int async_cur, async_it;  // cur and it when step_async last began fresh
+  bool fresh;        // no step has been issued since the upload
+  // A step after the first needed the first-step passes: until the next
+  // upload every step chooses its dt with them (dt_each_step).
+  bool dt_passes;
+  int async_cur, async_it;  // cur and it at the upload (vacgpu_internal_step_async)
   // done and steps of the control block after each of the two chunks of
   // steps in flight (page-locked), and the events behind those copies
   int* poll;
@@ -193,10 +196,10 @@ struct vacgpu_handle {
   cudaEvent_t open_ev;
   int open_k;
   // fused mixed sweep: TMA descriptors of the two state buffers, 1/dx
-  // CUDA graphs of two consecutive steps, keyed by (state buffer, parity
-  // of it): replayed instead of re-issuing ~20 launches per step.
-  cudaGraphExec_t gexec[2][2];
-  long long glaunch[2][2][VACGPU_K_NCLASS];  // kernels per replay, by class
+  // CUDA graphs of two consecutive steps, keyed by (dt_passes, state buffer,
+  // parity of it): replayed instead of re-issuing ~20 launches per step.
+  cudaGraphExec_t gexec[2][2][2];
+  long long glaunch[2][2][2][VACGPU_K_NCLASS];  // kernels per replay, by class
   bool warmed;
   bool fused;
   CUtensorMap tmap[2][2];  // [state buffer][x/z sweeps, y sweep]
@@ -623,9 +626,10 @@ void run_sweep(vacgpu_handle* h, int d0, int d1) {
 
 // Every step chooses its dt with the passes of run_dt and ends with
 // launch_step_end where a user hook or the specialeta field takes part in
-// the choice; elsewhere launch_step_ctl ends a step and chooses the next
-// one's dt, and run_dt serves the first step after an upload.
-bool dt_each_step(const vacgpu_handle* h) { return h->dtsp_fn || h->etaf; }
+// the choice, or where a step after the first needed the passes (dt_passes);
+// elsewhere launch_step_ctl ends a step and chooses the next one's dt, and
+// run_dt serves the first step after an upload.
+bool dt_each_step(const vacgpu_handle* h) { return h->dtsp_fn || h->etaf || h->dt_passes; }
 
 // The dt choice with the first-step passes (each does nothing unless this
 // step needs it).
@@ -718,29 +722,20 @@ void begin_call(vacgpu_handle* h, int maxsteps, double tstop) {
   kbegin(h, VACGPU_K_CONTROL);
   launch_call_ctl(h->ctrl, h->p, maxsteps, tstop, !each && !h->fresh, h->st);
   kend(h);
-  if (!each && h->fresh && maxsteps > 0) {
-    run_dt_any(h);
-    h->fresh = false;
-  }
-}
-
-// After done = 4 with `steps` steps done of those issued from buffer cur0:
-// the passes of the pending step's dt choice.
-void resume_dt(vacgpu_handle* h, int cur0, int steps) {
-  const int nsw = h->p.dimsplit ? h->p.ndim : 1;
-  h->cur = cur0 ^ ((steps * nsw) & 1);
-  launch_resume(h->ctrl, h->st);
-  run_dt_any(h);
+  if (maxsteps == 0) return;
+  if (!each && h->fresh) run_dt_any(h);
+  h->fresh = false;
 }
 
 // Captured graphs hold the launch arguments and hooks of their capture.
 void drop_graphs(vacgpu_handle* h) {
-  for (int i = 0; i < 2; i++)
-    for (int j = 0; j < 2; j++)
-      if (h->gexec[i][j]) {
-        cudaGraphExecDestroy(h->gexec[i][j]);
-        h->gexec[i][j] = nullptr;
-      }
+  for (auto& mode : h->gexec)
+    for (auto& cur : mode)
+      for (cudaGraphExec_t& ex : cur)
+        if (ex) {
+          cudaGraphExecDestroy(ex);
+          ex = nullptr;
+        }
 }
 
 // Issue k steps on the handle's stream without waiting: two-step units
@@ -753,8 +748,8 @@ int issue_steps(vacgpu_handle* h, int k, int it_base) {
   for (int s = 0; s < k;) {
     const int par = (it_base + s) & 1;
     if (graphs && h->warmed && k - s >= 2) {
-      cudaGraphExec_t& ex = h->gexec[h->cur][par];
-      const int cur0 = h->cur;
+      const int cur0 = h->cur, mode = h->dt_passes;
+      cudaGraphExec_t& ex = h->gexec[mode][cur0][par];
       if (!ex) {
         cudaGraph_t gr;
         long long before[VACGPU_K_NCLASS];
@@ -770,13 +765,13 @@ int issue_steps(vacgpu_handle* h, int k, int it_base) {
         CK(cudaGraphInstantiate(&ex, gr, 0));
         cudaGraphDestroy(gr);
         for (int k = 0; k < VACGPU_K_NCLASS; k++) {
-          h->glaunch[cur0][par][k] = h->nlaunch[k] - before[k];
+          h->glaunch[mode][cur0][par][k] = h->nlaunch[k] - before[k];
           h->nlaunch[k] = before[k];  // counted when the graph runs
         }
         h->cur = cur0;
       }
       CK(cudaGraphLaunch(ex, h->st));
-      for (int k = 0; k < VACGPU_K_NCLASS; k++) h->nlaunch[k] += h->glaunch[cur0][par][k];
+      for (int k = 0; k < VACGPU_K_NCLASS; k++) h->nlaunch[k] += h->glaunch[mode][cur0][par][k];
       h->cur = cur0 ^ ((2 * nsw) & 1);
       s += 2;
     } else {
@@ -906,18 +901,22 @@ int vacgpu_internal_step_async(vacgpu_handle* h, int k) {
   return 0;
 }
 // After the steps of vacgpu_internal_step_async ran: how many of those
-// issued are still to do, because a step waits for the first-step passes
-// (every later call stops there as well; the next one issues the passes).
-// None are where not one ran since those passes: the run is finished.
-int vacgpu_internal_steps_left(vacgpu_handle* h, int* left) {
+// issued are still to do, because a step waits for the first-step passes.
+// Every later call would stop there as well; from here on each step has the
+// passes (dt_passes, also returned).
+int vacgpu_internal_steps_left(vacgpu_handle* h, int* left, int* passes) {
   int st[3];  // it, itmin, done
   CK(cudaMemcpyAsync(st, &h->ctrl->it, sizeof(st), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
-  *left = st[2] == 4 && st[0] != h->async_it ? h->it_host - st[0] : 0;
+  if (st[2] == 4) {
+    h->dt_passes = true;
+    h->warmed = false;  // its kernels run once before a graph captures them
+  }
+  *left = st[2] == 4 ? h->it_host - st[0] : 0;
+  *passes = h->dt_passes;
   h->it_host = st[0];
   const int nsw = h->p.dimsplit ? h->p.ndim : 1;
   h->cur = h->async_cur ^ (((st[0] - h->async_it) * nsw) & 1);
-  if (st[2] == 4) h->fresh = true;
   return 0;
 }
 void* vacgpu_internal_stream(vacgpu_handle* h) { return (void*)h->st; }
@@ -1365,6 +1364,7 @@ int vacgpu_upload(vacgpu_handle* h, const double* w, int it, double t) {
   if (h->hook_failed) return fail("the specialbound hook failed");
   h->cur = 0;
   h->fresh = true;
+  h->dt_passes = false;
   h->it_host = it;
   h->have_state = true;
   return 0;
@@ -1460,12 +1460,14 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
   if (h->etaf && !h->eta_fn) return fail(NO_ETA);
   const int nsw = h->p.dimsplit ? h->p.ndim : 1;
   const int start_cur = h->cur;
-  begin_call(h, maxsteps, tstop);
-  CK(cudaGetLastError());
   // Steps are issued in chunks, two in flight, so the device does not wait
   // for the host between chunks; each chunk's done flag is read back behind
-  // it, and no more are issued once one reports a stop.
-  int issued = 0, head = 0, inflight = 0, chunk = STEP_CHUNK;
+  // it, and no more are issued once one reports a stop.  The first chunks
+  // after an upload are short: where the second step waits for the first-step
+  // passes, few are issued in vain.
+  int issued = 0, head = 0, inflight = 0, chunk = h->fresh ? 2 : STEP_CHUNK;
+  begin_call(h, maxsteps, tstop);
+  CK(cudaGetLastError());
   Ctrl c;
   while (true) {
     bool stop = false;
@@ -1473,6 +1475,7 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
       const int k = maxsteps - issued < chunk ? maxsteps - issued : chunk;
       if (issue_steps(h, k, h->it_host + issued)) return 1;
       issued += k;
+      if (chunk < STEP_CHUNK) chunk *= 2;
       CK(cudaGetLastError());
       if (h->hook_failed) {
         h->hook_failed = false;
@@ -1500,11 +1503,16 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
     CK(cudaStreamSynchronize(h->st));
     inflight = 0;
     if (c.done != 4) break;
-    // a step later than the first needs the first-step passes: run them,
-    // and go on from the steps done, one at a time
-    resume_dt(h, start_cur, c.steps);
+    // A step later than the first needs the first-step passes (gas with no
+    // wave speed along one axis does at every step): go on from the steps
+    // done, each step with its passes.  500 steps of gas without pressure that
+    // flows along x, in FP64: 30 ms on 64^2 (a host round trip for each step's
+    // passes took 71; ordinary gas takes 26), 60 on 256^2 (97; 49).
+    h->dt_passes = true;
+    h->warmed = false;  // its kernels run once before a graph captures them
+    h->cur = start_cur ^ ((c.steps * nsw) & 1);
     issued = c.steps;
-    chunk = 1;
+    launch_resume(h->ctrl, h->st);
   }
   // every executed step swapped the buffers nsw times; skipped ones none
   h->cur = start_cur ^ ((c.steps * nsw) & 1);
@@ -1676,9 +1684,7 @@ void vacgpu_destroy(vacgpu_handle* h) {
     if (e) cudaEventDestroy(e);
   drain_events(h);
   for (auto e : h->pool) cudaEventDestroy(e);
-  for (int i = 0; i < 2; i++)
-    for (int j = 0; j < 2; j++)
-      if (h->gexec[i][j]) cudaGraphExecDestroy(h->gexec[i][j]);
+  drop_graphs(h);
   if (h->own_st) cudaStreamDestroy(h->own_st);
   delete h;
 }
