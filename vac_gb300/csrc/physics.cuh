@@ -235,8 +235,9 @@ __device__ __forceinline__ double limiter_fn(int lim, double a, double b) {
 // 64-bit integers, doubles of clear sign bit compare as their values do, and
 // where a and b differ in sign the result is zero.  What is left for the
 // FP64 pipe is woodward's (a+b)/4 or minmod's factor 1/2, of 8 to 10
-// operations (comparisons run there as well).  NaN and slopes that overflow
-// take limiter_fn itself.
+// operations (comparisons run there as well).  NaN in either operand and
+// slopes that overflow take limiter_fn itself (what minmod gives for a NaN a
+// and a finite b is finite, and is not left to how the selects compile).
 static __device__ __noinline__ double half_limiter_fn(int lim, double a, double b) {
   return 0.5 * limiter_fn(lim, a, b);
 }
@@ -261,8 +262,8 @@ __device__ __forceinline__ double hlimiter_fn(int lim, double a, double b) {
   if (lim == LIM_MINMOD) {
     long long r = xa < xb ? xa : xb;
     if (xb < 0) r = xb == SIGN ? SIGN : 0;
-    return (xb & ~SIGN) <= INF ? 0.5 * __longlong_as_double(r ^ sg)
-                               : half_limiter_fn(lim, a, b);
+    return xa <= INF && (xb & ~SIGN) <= INF ? 0.5 * __longlong_as_double(r ^ sg)
+                                            : half_limiter_fn(lim, a, b);
   }
   return half_limiter_fn(lim, a, b);
 }
