@@ -353,3 +353,124 @@ def test_fused_gas_3d(gpu_lib, monkeypatch, name, nx, lim, bc):
     test_fused_against_oracle_and_split(
         gpu_lib, monkeypatch, name, lambda: _hd3(nx), lim, bc, 8,
         (lambda p: reflecting(p, 3)) if bc == "symm" else None)
+
+
+LONG_ITEMS = [
+    # items of 2 rows and a last one of one row; of 4 and one; of 16 and 13
+    ("mhd-600x131-reflect", lambda: _ot_shape(600, 131), "minmod", "symm", 4,
+     lambda p: reflecting(p, 2)),
+    ("hd-700x777-cont", lambda: _hd(700, 777), "woodward", "cont", 3, None),
+    ("mhd-1210x1101-periodic", lambda: _ot_shape(1210, 1101), "woodward", "periodic", 2, None),
+]
+
+
+@pytest.mark.parametrize("name,mk,lim,bc,n,tweak", LONG_ITEMS, ids=[c[0] for c in LONG_ITEMS])
+def test_line_sweep_items_of_several_rows(gpu_lib, monkeypatch, name, mk, lim, bc, n, tweak):
+    """2-D grids with more rows than warps, whose work items march several
+    rows (the shapes above have items of one row) and end on a shorter item,
+    against the oracle and the split kernels."""
+    test_fused_against_oracle_and_split(gpu_lib, monkeypatch, name, mk, lim, bc, n, tweak)
+
+
+@pytest.mark.parametrize("nx,lim,bc", [((600, 131), "woodward", "cont"),
+                                       ((600, 131), "minmod", "symm"),
+                                       ((601, 400), "minmod", "periodic")])
+def test_line_sweep_roe_items_of_several_rows(gpu_lib, monkeypatch, nx, lim, bc):
+    test_fused_roe_against_oracle_and_split(gpu_lib, monkeypatch, "rows", nx, lim, bc, {})
+
+
+@pytest.mark.parametrize("lim", ["minmod", "woodward"])
+@pytest.mark.parametrize("roe", [False, True])
+def test_rows_per_item_are_invisible(gpu_lib, roe, lim):
+    """A periodic 61x50 state repeated along y: 26 copies run in items of three
+    rows, one copy in items of one, and each copy keeps the bits.  (Cells of
+    1/64, so that every cell width is exact at either height.)"""
+    s = inistate.random_modes(64, seed=9, p0=0.5, ndim=2)
+    w = s.w[:, :61, :50]
+    out = []
+    for k in (1, 26):
+        x = np.stack(np.meshgrid((np.arange(61) + 0.5) / 64, (np.arange(50 * k) + 0.5) / 64,
+                                 indexing="ij"))
+        t = inistate._snap(x, np.ascontiguousarray(np.tile(w, (1, 1, k))), 5.0 / 3.0, True, 2,
+                           "repeated modes")
+        p = inistate.params_for(t, limiter=lim, precision=abi.PREC_MIXED)
+        if roe:
+            p.typefull = abi.TVDMU
+        e = Engine(p, t.x, t.w)
+        e.step(6)
+        assert e.kernel_stats()["sweep"][0] == 12
+        out.append((e.t, e.state()))
+        e.close()
+    assert out[0][0] == out[1][0]
+    many = np.ascontiguousarray(np.tile(out[0][1], (1, 1, 26)))
+    assert np.array_equal(many.view(np.uint64), out[1][1].view(np.uint64))
+
+
+@pytest.mark.parametrize("nx,lim,bc", [((33, 33, 33), "minmod", "symm"),
+                                       ((64, 50, 41), "woodward", "periodic"),
+                                       ((97, 88, 90), "minmod", "cont")])
+def test_z_chunk_of_roe_sweeps_is_invisible(gpu_lib, monkeypatch, nx, lim, bc):
+    s = inistate.random_modes(max(nx), seed=6, p0=0.5)
+    s.x = inistate.domain_grid(nx, (0.0,) * 3, tuple(n / max(nx) for n in nx))
+    s.w = np.ascontiguousarray(s.w[:, :nx[0], :nx[1], :nx[2]])
+    s.nx = nx
+    p = inistate.params_for(s, limiter=lim, bc=bc, precision=abi.PREC_MIXED)
+    p.typefull = abi.TVDMU
+    if bc == "symm":
+        reflecting(p, 3)
+    n = 2 if bc == "symm" else 5
+    out = []
+    for pin in (None, "5", "32"):
+        if pin:
+            monkeypatch.setenv("VACGPU_NZC", pin)
+        e = Engine(p, s.x, s.w)
+        e.step(n)
+        assert e.kernel_stats()["sweep"][0] == 3 * n
+        out.append((e.t, e.state()))
+        e.close()
+    for t, w in out[1:]:
+        assert t == out[0][0] and np.array_equal(w.view(np.uint64), out[0][1].view(np.uint64))
+
+
+ROE_FORMS = [
+    ("rm3-stretched", (24, 33, 18), "woodward", "stretched"),
+    ("rm2-stretched", (70, 50), "minmod", "stretched"),
+    ("rm3-gravity", (24, 33, 18), "minmod", "gravity"),
+    ("rm2-gravity", (70, 50), "woodward", "gravity"),
+]
+
+
+@pytest.mark.parametrize("name,nx,lim,form", ROE_FORMS, ids=[c[0] for c in ROE_FORMS])
+def test_fused_roe_on_stretched_grids_and_with_gravity(gpu_lib, monkeypatch, name, nx, lim, form):
+    """The fused Roe flux takes |a| without the factor dt*2/(dx(i)+dx(j)) that
+    the split kernels multiply by and divide out again: on cells whose widths
+    vary, and with the gravity source, against the oracle and the split
+    kernels (bounds as for the other Roe cases)."""
+    nd = len(nx)
+    s = inistate.random_modes(max(nx), seed=8, p0=0.5, ndim=nd)
+    s.x = inistate.domain_grid(nx, (0.0,) * nd, tuple(n / max(nx) for n in nx))
+    s.w = np.ascontiguousarray(s.w[(slice(None),) + tuple(slice(0, n) for n in nx)])
+    s.nx = nx
+    if form == "stretched":
+        s = inistate.stretched(s)
+    p64 = inistate.params_for(s, limiter=lim)
+    pm = inistate.params_for(s, limiter=lim, precision=abi.PREC_MIXED)
+    p64.typefull = pm.typefull = abi.TVDMU
+    g = [0.3, -0.2, 0.1][:nd]
+    o = Oracle(p64, s.x, s.w)
+    if form == "gravity":
+        o.register_source(abi.SRC_GRAVITY, g)
+    o.step(8)
+    out = []
+    for fused in ("1", "0"):
+        monkeypatch.setenv("VACGPU_FUSED", fused)
+        e = Engine(pm, s.x, s.w)
+        if form == "gravity":
+            e.register_source(abi.SRC_GRAVITY, g)
+        e.step(8)
+        assert (e.kernel_stats()["sweep"][0] > 0) == (fused == "1")
+        assert abs(e.t - o.t) <= 1e-6 * o.t
+        out.append(e.state())
+        assert max(rel_l1(out[-1], o.state())) <= MIXED_REL_L1
+        e.close()
+    assert max(rel_l1(out[0], out[1])) <= 2 * FUSED_VS_SPLIT
