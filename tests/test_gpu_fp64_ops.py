@@ -1,6 +1,6 @@
-"""The FP64 path's quotient by a shared reciprocal and its half slopes on the
-integer ALUs, operand by operand: the bits of a/b and of 0.5*limiter, over
-random bit patterns, neighbouring mantissas, the exponents at which the
+"""The FP64 path's quotient by a shared reciprocal, its half slopes on the
+integer ALUs and its folded halves, operand by operand: the bits of a/b, of
+0.5*limiter and of 0.5*a + b, over random bit patterns, neighbouring mantissas, the exponents at which the
 quotient changes over to a plain division, subnormals, zeros of either sign,
 infinities and NaN."""
 import ctypes as C
@@ -29,7 +29,7 @@ def _ops(a, b):
     f = C.CDLL(so).fp64_ops
     dp = C.POINTER(C.c_double)
     f.argtypes = [dp, dp, dp, C.c_longlong]
-    out = np.empty((8, a.size))
+    out = np.empty((10, a.size))
     assert f(*(v.ctypes.data_as(dp) for v in (a, b, out)), a.size) == 0
     return out
 
@@ -64,7 +64,7 @@ def _operands(kind):
 def test_quotient_and_half_slopes(gpu_lib, kind):
     a, b = _operands(kind)
     out = _ops(a, b)
-    for k, what in ((0, "quotient"), (2, "minmod"), (4, "woodward")):
+    for k, what in ((0, "quotient"), (2, "minmod"), (4, "woodward"), (8, "half plus")):
         got, ref = out[k], out[k + 1]
         bad = ~((got.view(np.uint64) == ref.view(np.uint64)) | (np.isnan(got) & np.isnan(ref)))
         assert not bad.any(), (what, a[bad][:3], b[bad][:3], got[bad][:3], ref[bad][:3])

@@ -573,3 +573,20 @@ def test_fp64_nan_cells_spread_as_the_oracle_s(gpu_lib):
                     got, ref = np.isnan(e.state()), np.isnan(o.state())
                     assert ref.any() and np.array_equal(got, ref), (nx, mhd, lim, full)
                 e.close()
+
+
+def test_fp64_front_into_gas_at_rest_keeps_subnormal_bits(gpu_lib):
+    """A hot sphere in magnetised gas at rest: ahead of its front the momenta
+    and B fall off to the subnormal range within the run, where halving
+    rounds: bit for bit the oracle's state, the last subnormal bit included."""
+    nx = (96, 90, 88)
+    x = inistate.domain_grid(nx, (-0.5,) * 3, (0.5,) * 3)
+    pr = np.where(np.sqrt(sum(c * c for c in x)) < 0.1, 10.0, 0.1)
+    z = np.zeros(nx)
+    s = inistate._snap(x, inistate.conserve_mhd(z + 1.0, [z] * 3, pr, [z + 0.5, z, z], 5.0 / 3.0),
+                       5.0 / 3.0, True, 3, "hot sphere")
+    o, e = run_both(s, "woodward", "cont", 25)
+    got, ref = e.state(), o.state()
+    tiny = (ref != 0) & (np.abs(ref) < np.finfo(np.float64).tiny)
+    assert tiny.sum() > 1000
+    assert e.t == o.t and np.array_equal(bits(got), bits(ref)), int((bits(got) != bits(ref)).sum())

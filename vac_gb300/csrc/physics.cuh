@@ -6,9 +6,12 @@
 // contraction for the FP64 path), so each value is bit-identical to the CPU
 // restatement.  A factor that is a power of two is folded into an FMA where
 // the reference multiplies by it and adds: the product is exact, so the
-// FMA rounds once, where the reference's sum does (every result above the
-// subnormal range keeps its bits, and the FP64 pipe, which bounds these
-// kernels, issues one operation less).  Variable layout (src/vacpar.t.mhd:9-26, src/vacpar.t.hd:9-26):
+// FMA rounds once, where the reference's sum does, and the FP64 pipe, which
+// bounds these kernels, issues one operation less.  A half is not exact in
+// the subnormal range, which the fluxes and div B reach ahead of a front that
+// spreads into gas at rest (half_plus); the pressure and the fast speed halve
+// and quarter terms that are added to others of ordinary size.  Variable
+// layout (src/vacpar.t.mhd:9-26, src/vacpar.t.hd:9-26):
 //   rho=0, m_c=c (c=1..NDIR), e=NDIR+1, b_c=NDIR+1+c.
 #pragma once
 #include <cuda_runtime.h>
@@ -69,6 +72,17 @@ __device__ __forceinline__ double div64(double a, const Rcp64& r) {
   if (!(r.ok && exponent_within(a, 800)))
     q = r.ok && (__double_as_longlong(a) << 1) == 0 ? a : div_any(a, r.b);
   return q;
+}
+
+// 0.5*s may round: s is not zero and its half is subnormal
+__device__ __forceinline__ bool half_rounds(double s) {
+  const unsigned hi = (unsigned)__double2hiint(s) << 1;
+  return hi < 0x00400000u && (hi | (unsigned)__double2loint(s)) != 0;
+}
+// 0.5*s + d with the product rounded first, as the reference has it
+static __device__ __noinline__ double half_plus_any(double s, double d) { return 0.5 * s + d; }
+__device__ __forceinline__ double half_plus(double s, double d) {
+  return half_rounds(s) ? half_plus_any(s, d) : fma(0.5, s, d);
 }
 
 // getptotal, src/vacphys0.t.mhd:225-257 (unclipped total pressure)

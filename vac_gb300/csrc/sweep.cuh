@@ -242,10 +242,14 @@ struct Sweep {
       for (int d = 0; d < NDIM; d++) {
         const T* q = wct + (long long)(L::B0 + 1 + d) * a.g.vs;
         const R df = R(q[st[d]]) - R(q[-st[d]]);
-        if constexpr (sizeof(R) == 8)  // divb + 0.5*df/dx
-          divb = fma(0.5, PH::div_dx(df, a.a, d, c[d]), divb);
-        else
+        if constexpr (sizeof(R) == 8) {  // divb + 0.5*df/dx
+          const R q = PH::div_dx(df, a.a, d, c[d]);
+          divb = half_rounds(df) || half_rounds(q)
+                     ? divb + PH::div_dx(0.5 * df, a.a, d, c[d])
+                     : fma(0.5, q, divb);
+        } else {
           divb = divb + R(0.5) * df / PH::dx(a.a, d, c[d]);
+        }
       }
       divb = PH::qdiv(qdt) * divb;
       const typename PH::Den ir = PH::den(wc[0]);
@@ -517,7 +521,7 @@ struct Sweep {
     for (int iw = 0; iw < NW; iw++) {
       const R diss = -cmax * R(0.5) * (wR[iw] - wL[iw]);
       if constexpr (sizeof(R) == 8)
-        F[iw] = fma(0.5, fL[iw] + fR[iw], diss);
+        F[iw] = half_plus(fL[iw] + fR[iw], diss);
       else
         F[iw] = R(0.5) * (fL[iw] + fR[iw]) + diss;
     }
