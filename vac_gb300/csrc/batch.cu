@@ -514,7 +514,7 @@ int autotune(vacgpu_batch* b) {
     return 0;
   };
   if (copy(true)) return 1;
-  int sms = 152;
+  int sms = NUM_SMS;
   {
     int dev = 0;
     cudaGetDevice(&dev);

@@ -205,7 +205,7 @@ __global__ void k_eta_max(SweepArgs a, int first_only) {
 
 void launch_eta_max(const SweepArgs& a, int first_only, cudaStream_t st) {
   k_eta_reset<<<1, 1, 0, st>>>(a.ctrl, first_only);
-  k_eta_max<<<2 * 152, 256, 0, st>>>(a, first_only);
+  k_eta_max<<<2 * NUM_SMS, 256, 0, st>>>(a, first_only);
 }
 
 void launch_set_qt(Ctrl* c, int mode, cudaStream_t st) {

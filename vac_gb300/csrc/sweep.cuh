@@ -1142,12 +1142,12 @@ inline unsigned grid_for(long long n, int nt) {
 }
 
 // Threads per block of the predictor, face and cell passes: one warp where
-// blocks of four would be fewer than eight per SM (152), so the last blocks
+// blocks of four would be fewer than eight per SM, so the last blocks
 // leave no SM idle while others run two -- and a grid of few cells is spread
 // over more SMs (the FP64 pipe of one SM takes 6 us for the faces of 128
 // cells).  With that and the ghost images in the passes a 200^2 MHD step in
 // FP64 takes 125 us (158 before), one of 100 cells in 1-D 25 us (29).
-inline int split_threads(long long n) { return n < 8LL * 152 * 128 ? 32 : 128; }
+inline int split_threads(long long n) { return n < 8LL * NUM_SMS * 128 ? 32 : 128; }
 
 template <class PH>
 struct Launch {
@@ -1304,9 +1304,6 @@ struct Launch {
   }                                                                          \
   void launch_ghost_##SUF(const SweepArgs& s, PH::T* w, cudaStream_t st) {   \
     Launch<PH>::ghost(s, w, st);                                             \
-  }                                                                          \
-  void launch_ghost_yz_##SUF(const SweepArgs& s, PH::T* w, cudaStream_t st) { \
-    Launch<PH>::ghost(s, w, st, true);                                       \
   }                                                                          \
   void launch_source_pass_##SUF(const SweepArgs& s, const PH::T* wct,        \
                                 const PH::T* w, PH::T* wout, int pred,       \

@@ -125,7 +125,6 @@ bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win, 
   const int am = kind == 2 ? s.d0 : 2;
   dim3 grid((s.g.nx[0] + tx - 1) / tx, (s.g.nx[ar] + ty - 1) / ty,
             nd == 3 ? (s.g.nx[am] + nzc - 1) / nzc : 1);
-  a.zchunks = grid.z;
   const CUtensorMap* map = (const CUtensorMap*)tmap;
   const int D = s.d0;
 #define L1(ND, DD)                                              \

@@ -94,7 +94,6 @@ struct FusedArgs {
   Ctrl* ctrl;
   float* wout;
   int nzc;               // planes per CTA (3-D)
-  int zchunks;
   int periodic_mask[3];  // bit iw set: variable iw periodic in dimension d
   int asymm_lo[3], asymm_hi[3];  // bit iw set: 'asymm' at that face
   float gravf[3];        // gravity source parameters (FP32)
@@ -544,11 +543,6 @@ struct Fused {
     return b;
   }
 
-  static __device__ __forceinline__ int preimages(const FusedArgs& a, int d, int gi, int& p1,
-                                                  int& f1, int& p2) {
-    return ghost_preimages(a.g, a.ph, d, gi, p1, f1, p2);
-  }
-
   // getboundary of the new state, done by its sources: every ghost cell
   // (gx, gy, gz) holds sign * w(map_x(gx), map_y(gy), map_z(gz)) (the
   // region-by-region copies of src/vacgrid.t:195-413 composed), so the cell
@@ -564,7 +558,7 @@ struct Fused {
                                                       const float (&acc)[NW]) {
     const DevGrid& g = a.g;
     int x1, x2, fx;
-    const int nx_ = 1 + preimages(a, 0, gc[0], x1, fx, x2);
+    const int nx_ = 1 + ghost_preimages(a.g, a.ph, 0, gc[0], x1, fx, x2);
     const bool yin = NDIM < 2 || (gc[1] >= 4 && gc[1] < g.nx[1]);
     const bool zin = NDIM < 3 || (gc[2] >= 4 && gc[2] < g.nx[2]);
     if (yin && zin) {
@@ -578,8 +572,8 @@ struct Fused {
       return;
     }
     int y1 = 0, y2 = 0, fy = 0, z1 = 0, z2 = 0, fz = 0;
-    const int ny_ = NDIM > 1 ? 1 + preimages(a, 1, gc[1], y1, fy, y2) : 1;
-    const int nz_ = NDIM > 2 ? 1 + preimages(a, 2, gc[2], z1, fz, z2) : 1;
+    const int ny_ = NDIM > 1 ? 1 + ghost_preimages(a.g, a.ph, 1, gc[1], y1, fy, y2) : 1;
+    const int nz_ = NDIM > 2 ? 1 + ghost_preimages(a.g, a.ph, 2, gc[2], z1, fz, z2) : 1;
 #pragma unroll 1
     for (int k = 0; k < nz_; k++) {
       const int pz = k == 0 ? gc[2] : (k == 1 ? z1 : z2);

@@ -32,8 +32,9 @@ __global__ void __launch_bounds__(L2_NT, MHD ? 2 : 4)
 // Batched grids: each warp takes items gw, gw + W, ... of the work list
 // (W warps in the launch); an item is (grid, strip bx, output rows by ..
 // bz-1 in ghost-range indices).
-// (register bound: the work-list loop of the general y sweep needs more than
-// 128 registers, so it runs three CTAs per SM rather than spill)
+// (register bound: the work-list loop of the general y sweep needs some 160
+// registers, so it runs three CTAs per SM; the others keep four at 128, with
+// 8 to 20 bytes spilled in the general x and the periodic y sweep)
 template <int D, bool MHD, int LIMC, bool GEN>
 __global__ void __launch_bounds__(L2_NT, MHD ? 2 : (D == 1 && GEN ? 3 : 4))
     kb_sweep_line2(const BItem* __restrict__ items, int nitems, const BInst* __restrict__ insts,
@@ -71,17 +72,21 @@ bool line2_applies(const FusedArgs& a, bool mhd) {
 
 // Rows per work item of a single grid: the fewest that keep the items within
 // the warps resident at once (four a CTA; two CTAs per SM for MHD, four for
-// HD, 152 SMs), at most L2_ROWS_MAX.  A grid that fits in one wave is bound
-// by the march of one item -- 1.6 us a row, whatever the other warps do --
-// so short items win although each predicts up to three rows beyond its own:
-// a 128^2 MHD sweep takes 12 us in items of 1 row, 64 us in items of 32
-// (512^2: 20 us with 4 rows, 64 with 32; 1001^2: 46 with 16, 64 with 32).
-// Larger grids run several waves: 16 rows took 128 us at 2048^2, 32 rows
-// 130, 8 rows 133.
+// HD), at most L2_ROWS_MAX.  A grid that fits in one wave is bound by the
+// march of one item -- 1.4 us a row of MHD, whatever the other warps do -- so
+// short items win although each predicts up to three rows beyond its own.  us
+// a sweep of periodic grids by rows per item, the rule's choice first:
+//   MHD   128^2 10.6 (1; 4: 15, 32: 54)    512^2 17.8 (4; 1: 28, 32: 54)
+//        1001^2 39.7 (15; 8: 42, 32: 57)  2048^2 121 (16; 8: 128, 32: 121)
+//   Roe   128^2 11.3 (1; 4: 16, 32: 59)    512^2 19.4 (4; 1: 31, 32: 59)
+//        1001^2 43.8 (15; 8: 47, 32: 62)  2048^2 139 (16; 8: 146, 32: 139)
+//   gas   128^2  9.3 (1; 4: 12, 32: 41)    512^2 14.9 (2; 4: 13.7, 32: 41)
+//        1001^2 24.9 (7; 16: 31, 32: 44)  2048^2 65.9 (16; 8: 66, 32: 72)
+// and with outflow faces likewise.
 constexpr int L2_ROWS_MAX = 16;
 static int line2_rows(int D, bool mhd, const DevGrid& g) {
   const int strips = line2_strips(D, mhd, g.nx[0]);
-  const int warps = 152 * (mhd ? 2 : 4) * (L2_NT / 32);
+  const int warps = NUM_SMS * (mhd ? 2 : 4) * (L2_NT / 32);
   int rows = 1;
   while (rows < L2_ROWS_MAX && strips * ((g.nx[1] + rows - 1) / rows) > warps) rows++;
   return rows;
@@ -231,7 +236,10 @@ __device__ __forceinline__ bool grid_sync(GridSync* gs, unsigned nb,
 // Line2::run and the first-step passes use ld.global.cg), and the rows of
 // the state arrive by cp.async.cg, so no stale L1 line from an earlier step
 // is read.  (HD: four CTAs per SM at 128 registers; on 64 uneven HD grids
-// that ran about 3 % faster than three CTAs per SM.)
+// that ran about 3 % faster than three CTAs per SM.  The general form spills
+// 40 bytes there since the ghost images go out as pairs, and is faster all the
+// same: 40 steps of 64 grids with outflow faces take 15.4 ms, 16.1 when the
+// images went cell by cell and nothing spilled.)
 template <bool MHD, int LIMC, bool GEN>
 __global__ void __launch_bounds__(L2_NT, MHD ? 2 : 4) kb_steps_line2(const Line2Steps ls) {
   constexpr int RF = line2_ring_floats(MHD ? 6 : 4);

@@ -14,4 +14,8 @@ VACGPU_DEFINE_LAUNCHERS(mixed, PHff)
 VACGPU_DEFINE_LAUNCHERS(mixedf64, PHf64)
 VACGPU_DEFINE_LAUNCHERS(mixedf32, PHf32)
 
+void launch_ghost_yz_mixed(const SweepArgs& s, float* w, cudaStream_t st) {
+  Launch<PHff>::ghost(s, w, st, true);
+}
+
 }  // namespace vacgpu

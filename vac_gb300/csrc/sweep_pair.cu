@@ -44,21 +44,27 @@ bool pair_applies(const FusedArgs& a, bool mhd) {
 
 // Planes per CTA (z chunk) of a sweep over `tiles` column tiles and n planes
 // where the caller fixes none: the longest of 24, 20, 16 and 12 planes that
-// gives at least three waves (456 CTAs, three per SM, each), else the longest
-// of at most 8 that gives 350 CTAs, down to 2.  Every chunk predicts two
-// planes beyond its own, but the march of one CTA is a serial chain (1.9 us a
-// plane alone on its SM, 2.8 beside two others), so a small grid wants many
-// short ones, and a large one enough of them that the last wave leaves few
-// slots idle.  Measured, us a sweep (periodic MHD): 64^3 26.9 with 4 planes,
-// 32.7 with 8 (131 with 32 at an earlier state of the kernel); 96^3 53 with 8,
-// 62 with 16; 128^3 96 with 8, 104 with 16, 119 with 32; 160^3 154 with 12,
-// 163 with 16; 192^3 240 with 20, 252 with 28, 283 with 64; 256^3 513 with
-// 24, 529 with 32, 563 with 64; 320^3 942 with 24, 992 with 64.  (A trial of
-// each chunk in a grid's first call, before, cost that call six steps and
-// found nothing better than this by more than 2 %.)
+// gives at least three waves of three CTAs per SM, else the longest of at most
+// 8 that gives 350 CTAs, down to 2.  Every chunk predicts two planes beyond
+// its own, but the march of one CTA is a serial chain (1.9 us a plane alone on
+// its SM, 2.8 beside two others), so a small grid wants many short ones, and a
+// large one enough of them that the last wave leaves few slots idle.  The
+// thresholds come from the TVDLF MHD kernel; Roe's, which runs two CTAs per
+// SM, and gas's want nearly the same chunks.  us a sweep of periodic grids by
+// planes per CTA, the rule's choice first:
+//   MHD  64^3 26.6 (3-4; 8: 33, 32: 88)      128x113x120 86 (8; 16: 88, 32: 108)
+//       192^3 240 (20; 8: 254, 64: 283)           256^3 513 (24; 12: 525, 64: 558)
+//   Roe  64^3 31.8 (3-4; 4: 29, 32: 83)      128x113x120 99.6 (8; 16: 98, 32: 110)
+//       192^3 295 (20; 8: 316, 32: 305)           256^3 639 (24; 12: 661, 32: 649)
+//   gas  64^3 17.0 (3-4; 8: 20, 32: 50)      128x113x120 46.6 (8; 16: 46, 32: 61)
+//       192^3 128 (20; 8: 133, 64: 145)           256^3 263 (24; 12: 267, 64: 297)
+// With outflow faces likewise; over 48^3 to 320x300x310 no other chunk was
+// faster by more than 3 % for MHD and gas, or 2 % for Roe but for the 64^3
+// above.  (A trial of each chunk in a grid's first call, before, cost that
+// call six steps and gained nothing.)
 static int pair_chunk(int tiles, int n) {
   for (int z : {24, 20, 16, 12})
-    if ((long long)tiles * ((n + z - 1) / z) >= 3 * 456) return z;
+    if ((long long)tiles * ((n + z - 1) / z) >= 3 * 3 * NUM_SMS) return z;
   for (int z : {8, 6, 4, 3})
     if ((long long)tiles * ((n + z - 1) / z) >= 350) return z;
   return 2;

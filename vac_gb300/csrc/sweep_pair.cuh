@@ -240,8 +240,11 @@ __device__ __forceinline__ f2 p_hlim(f2 a, f2 b, const PairK& k) {
 // the x faces, and the caller fills the y and z layers.  The loops over the
 // images of the general index maps make the CTAs at a face, and with them the
 // sweep, slower than a fill of the y and z layers behind it (9 us at 128^3, 11
-// at 192^3) -- with outflow faces 128^3 took 129 us, 112 now -- so single
-// grids leave them out; a batch, which has no fill, keeps them.
+// at 192^3) -- with outflow faces 128^3 took 134 us, 112 now -- so single
+// grids leave them out; a batch, which has no fill, keeps them (150 to 230
+// bytes spilled in its general MHD form; 10 steps of eight grids of 48^3 to
+// 128^3 with outflow faces 17.2 ms, 20.4 with images cell by cell and fewer
+// spills, periodic ones 10.9 and 13.7).
 template <int D, bool MHD, int LIMC, bool GEN, bool ROE = false, bool IMG = true>
 struct PairSweep {
   static constexpr int K = D == 0 ? 0 : 2;        // in-plane / marching

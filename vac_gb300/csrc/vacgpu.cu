@@ -163,8 +163,8 @@ struct vacgpu_handle {
   // upload every step chooses its dt with them (dt_each_step).
   bool dt_passes;
   int async_cur, async_it;  // cur and it at the upload (vacgpu_internal_step_async)
-  // done and steps of the control block after each of the two chunks of
-  // steps in flight (page-locked), and the events behind those copies
+  // done of the control block after each of the two chunks of steps in
+  // flight (page-locked), and the events behind those copies
   int* poll;
   cudaEvent_t poll_ev[2];
   double* dx[3];
@@ -1487,15 +1487,15 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
       if (!h->poll) {
         for (cudaEvent_t& e : h->poll_ev)
           if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        CK(cudaMallocHost(&h->poll, 4 * sizeof(int)));
+        CK(cudaMallocHost(&h->poll, 2 * sizeof(int)));
       }
       const int slot = (head + inflight) & 1;
-      CK(cudaMemcpyAsync(h->poll + 2 * slot, &h->ctrl->done, 2 * sizeof(int),
+      CK(cudaMemcpyAsync(h->poll + slot, &h->ctrl->done, sizeof(int),
                          cudaMemcpyDeviceToHost, h->st));
       CK(cudaEventRecord(h->poll_ev[slot], h->st));
       if (++inflight < 2) continue;
       CK(cudaEventSynchronize(h->poll_ev[head]));
-      stop = h->poll[2 * head] != 0;
+      stop = h->poll[head] != 0;
       head ^= 1;
       inflight--;
     }

@@ -21,6 +21,9 @@ enum {
 // over (a block writes slot blockIdx % NSLOT); the step kernel folds them.
 constexpr int NSLOT = 128;
 
+// SMs of a GB300: the rules that split a grid by its size count CTAs by it.
+constexpr int NUM_SMS = 152;
+
 // State layout in HBM: one padded box per variable (structure of arrays,
 // like VAC's w(ixG^T,nw)), x fastest.  A row holds the nG[0] cells of
 // ghost+mesh+ghost starting at column xpad, chosen so the first mesh cell
@@ -264,7 +267,6 @@ struct SweepArgs {
   void launch_correct_##SUF(const SweepArgs& s, const T* w, const T* w1,     \
                             const T* base, T* wout, cudaStream_t st);        \
   void launch_ghost_##SUF(const SweepArgs& s, T* w, cudaStream_t st);        \
-  void launch_ghost_yz_##SUF(const SweepArgs& s, T* w, cudaStream_t st);     \
   void launch_source_pass_##SUF(const SweepArgs& s, const T* wct,            \
                                 const T* w, T* wout, int pred,               \
                                 cudaStream_t st);                            \
@@ -296,6 +298,8 @@ void launch_correct_roe_mixed(const SweepArgs& s, const float* w,
                               const float* w1, const float* base, float* wout,
                               cudaStream_t st);
 
+// the y and z ghost layers alone, behind a fused 3-D sweep
+void launch_ghost_yz_mixed(const SweepArgs& s, float* w, cudaStream_t st);
 // Fused single-kernel sweep of the mixed path (sweep_fused.cu): returns
 // false when no fused instance exists for the configuration.  `tmap` is the
 // CUtensorMap (as bytes) of the input state buffer with the box of the sweep
