@@ -474,3 +474,53 @@ def test_fused_roe_on_stretched_grids_and_with_gravity(gpu_lib, monkeypatch, nam
         assert max(rel_l1(out[-1], o.state())) <= MIXED_REL_L1
         e.close()
     assert max(rel_l1(out[0], out[1])) <= 2 * FUSED_VS_SPLIT
+
+
+def _superbee(nx, bc, mhd=True):
+    s = inistate.random_modes(max(nx), seed=6, p0=0.5)
+    s.x = inistate.domain_grid(nx, (0.0,) * 3, tuple(n / max(nx) for n in nx))
+    s.w = np.ascontiguousarray(s.w[:, :nx[0], :nx[1], :nx[2]])
+    s.nx = nx
+    if not mhd:
+        s = _hd3(nx, seed=6)
+    return s, inistate.params_for(s, limiter="superbee", bc=bc, precision=abi.PREC_MIXED)
+
+
+@pytest.mark.parametrize("nx,bc,mhd", [((33, 17, 33), "cont", True), ((64, 50, 41), "periodic", True),
+                                       ((31, 20, 9), "cont", False),
+                                       ((97, 88, 90), "periodic", False)])
+def test_z_chunk_of_the_one_cell_kernel_is_invisible(gpu_lib, monkeypatch, nx, bc, mhd):
+    """Limiters without a pair kernel: the chunk that a grid gets by its size
+    gives the bits of one pinned at 32."""
+    s, p = _superbee(nx, bc, mhd)
+    out = []
+    for pin in (None, "32"):
+        if pin:
+            monkeypatch.setenv("VACGPU_NZC", pin)
+        e = Engine(p, s.x, s.w)
+        e.step(4)
+        assert e.kernel_stats()["sweep"][0] == 12
+        out.append((e.t, e.state()))
+        e.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1].view(np.uint64), out[1][1].view(np.uint64))
+
+
+def test_z_chunk_of_the_one_cell_kernel_fits_the_grid(gpu_lib, monkeypatch):
+    """At 130x127x133 the size's chunk is no slower than the better of 8 and
+    16 planes by more than a tenth (32 planes: by 30 to 40 %)."""
+    s, p = _superbee((130, 127, 133), "cont")
+    us = {}
+    for pin in (None, "8", "16"):
+        if pin:
+            monkeypatch.setenv("VACGPU_NZC", pin)
+        e = Engine(p, s.x, s.w)
+        e.step(4)
+        for _ in range(3):
+            e.timing(True)
+            e.step(6)
+            n, ms = e.kernel_stats()["sweep"]
+            us[pin] = min(us.get(pin, 1e9), 1e3 * ms / n)
+        e.timing(False)
+        e.close()
+    assert us[None] <= 1.1 * min(us["8"], us["16"]), us

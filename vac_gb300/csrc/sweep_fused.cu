@@ -80,6 +80,32 @@ bool fused_roe_applies(const DevGrid& g, const DevPhys& ph, int ndir, bool mhd) 
   return g.ndim == 3 ? pair_applies(a, mhd) : g.ndim == 2 && line2_applies(a, mhd);
 }
 
+// Planes per CTA (z chunk) of the one-cell kernel over `tiles` column tiles
+// and n planes where the caller fixes none, as pair_chunk (sweep_pair.cu): the
+// longest that gives so many waves of two CTAs per SM, else the longest of at
+// most 8 that gives 250 CTAs, down to 2.  us a sweep by planes per CTA, the
+// rule's choice first (MHD vanleer periodic; superbee with outflow faces; gas,
+// vanleer with outflow faces):
+//   64^3         35 (4; 8: 44, 32: 126)    46 (59, 175)       32 (40, 112)
+//   128^3       165 (8; 12: 160, 32: 187) 200 (193, 246)     116 (111, 149)
+//   130x127x133 177 (12; 16: 194, 32: 239) 218 (230, 299)    127 (129, 172)
+//   192^3       437 (16-24; 12: 440, 32: 438) 520 (518, 549) 284 (282, 304)
+//   256^3       921 (24; 48: 914, 32: 929) 1052 (1068, 1084) 550 (577, 576)
+//   320x300x310 1538 (48; 24: 1584, 32: 1560) 1743 (1782, 1757)
+// A trial in a grid's first call, before 32 planes were taken for every grid,
+// found 169, 194, 437, 916 and 1544 (207, 231, 517, 1056 and 1748) from 128^3 on.
+static int fused_chunk(int tiles, int n) {
+  static const struct {
+    int z, waves;
+  } longer[] = {{48, 8}, {24, 4}, {16, 5}, {12, 3}};
+  auto ctas = [&](int z) { return (long long)tiles * ((n + z - 1) / z); };
+  for (const auto& l : longer)
+    if (ctas(l.z) >= l.waves * 2 * NUM_SMS) return l.z;
+  for (int z : {8, 6, 4, 3})
+    if (ctas(z) >= 250) return z;
+  return 2;
+}
+
 bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win, float* wout,
                         const float* const* idxf, int nzc, cudaStream_t st) {
   const int nd = s.g.ndim;
@@ -116,15 +142,15 @@ bool launch_sweep_fused(const SweepArgs& s, const void* tmap, const float* win, 
   if (nd == 2 && launch_sweep_line2(a, win, s.d0, s.mhd, st)) return true;
   // the one-cell kernel: tiles over x and the row axis, z chunks along the
   // marching axis
-  if (nzc <= 0) nzc = 32;
-  a.nzc = nzc;
   const int kind = fused_kind(nd, s.d0);
   const int tx = kind == 0 ? TileCfg<0>::TX : TileCfg<1>::TX;
   const int ty = kind == 1 ? TileCfg<1>::TY : TileCfg<0>::TY;
   const int ar = kind == 2 && s.d0 == 1 ? 2 : 1;
   const int am = kind == 2 ? s.d0 : 2;
-  dim3 grid((s.g.nx[0] + tx - 1) / tx, (s.g.nx[ar] + ty - 1) / ty,
-            nd == 3 ? (s.g.nx[am] + nzc - 1) / nzc : 1);
+  const int nxt = (s.g.nx[0] + tx - 1) / tx, nyt = (s.g.nx[ar] + ty - 1) / ty;
+  if (nzc <= 0) nzc = nd == 3 ? fused_chunk(nxt * nyt, s.g.nx[am]) : 1;
+  a.nzc = nzc;
+  dim3 grid(nxt, nyt, nd == 3 ? (s.g.nx[am] + nzc - 1) / nzc : 1);
   const CUtensorMap* map = (const CUtensorMap*)tmap;
   const int D = s.d0;
 #define L1(ND, DD)                                              \
