@@ -1462,20 +1462,20 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
   const int start_cur = h->cur;
   // Steps are issued in chunks, two in flight, so the device does not wait
   // for the host between chunks; each chunk's done flag is read back behind
-  // it, and no more are issued once one reports a stop.  The first chunks
-  // after an upload are short: where the second step waits for the first-step
-  // passes, few are issued in vain.
-  int issued = 0, head = 0, inflight = 0, chunk = h->fresh ? 2 : STEP_CHUNK;
+  // it, and no more are issued once one reports a stop.  (Shorter chunks after
+  // an upload, for gas whose second step waits for the first-step passes, cost
+  // every other call more than they spared that one: 72 steps of 576x668, mixed,
+  // take 3.50 ms, and 3.62 with chunks of 2, 4 and then 8.)
+  int issued = 0, head = 0, inflight = 0;
   begin_call(h, maxsteps, tstop);
   CK(cudaGetLastError());
   Ctrl c;
   while (true) {
     bool stop = false;
     while (issued < maxsteps && !stop) {
-      const int k = maxsteps - issued < chunk ? maxsteps - issued : chunk;
+      const int k = maxsteps - issued < STEP_CHUNK ? maxsteps - issued : STEP_CHUNK;
       if (issue_steps(h, k, h->it_host + issued)) return 1;
       issued += k;
-      if (chunk < STEP_CHUNK) chunk *= 2;
       CK(cudaGetLastError());
       if (h->hook_failed) {
         h->hook_failed = false;
@@ -1506,7 +1506,7 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
     // A step later than the first needs the first-step passes (gas with no
     // wave speed along one axis does at every step): go on from the steps
     // done, each step with its passes.  500 steps of gas without pressure that
-    // flows along x, in FP64: 30 ms on 64^2 (a host round trip for each step's
+    // flows along x, in FP64: 31 ms on 64^2 (a host round trip for each step's
     // passes took 71; ordinary gas takes 26), 60 on 256^2 (97; 49).
     h->dt_passes = true;
     h->warmed = false;  // its kernels run once before a graph captures them
