@@ -1462,10 +1462,10 @@ int vacgpu_step(vacgpu_handle* h, int maxsteps, double tstop, double* t,
   const int start_cur = h->cur;
   // Steps are issued in chunks, two in flight, so the device does not wait
   // for the host between chunks; each chunk's done flag is read back behind
-  // it, and no more are issued once one reports a stop.  (Shorter chunks after
-  // an upload, for gas whose second step waits for the first-step passes, cost
-  // every other call more than they spared that one: 72 steps of 576x668, mixed,
-  // take 3.50 ms, and 3.62 with chunks of 2, 4 and then 8.)
+  // it, and no more are issued once one reports a stop.  (Chunks of 2
+  // and 4 first after an upload, for gas whose second step waits for the
+  // first-step passes, gave a tube of 100 cells 3 % and cost larger grids more:
+  // 72 steps of 576x668, mixed, took 3.62 ms, 3.50 with chunks of 8.)
   int issued = 0, head = 0, inflight = 0;
   begin_call(h, maxsteps, tstop);
   CK(cudaGetLastError());
